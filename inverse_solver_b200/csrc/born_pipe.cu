@@ -9,11 +9,11 @@
 //
 //   * persistent CTAs (two per SM) walk the tiles of 16 x-lines (8 lines and
 //     three CTAs per SM for n = 200, 216); a tile of
-//     consecutive lines is one contiguous block of T, Field_n and Field, so
+//     consecutive lines is one contiguous block of T and of X, so
 //     one thread moves it into shared memory with bulk asynchronous copies
 //     (the TMA engine) completing on an mbarrier;
 //   * T of the next tile is copied while the current one is computed, and
-//     Field_n / Field of the next tile while the current one finishes its
+//     X of the next tile while the current one finishes its
 //     last FFT pass, so DRAM latency overlaps the FFT arithmetic instead of
 //     stalling it;
 //   * the plan is fixed at compile time: inverse radix-R2 pass (in place in
@@ -63,21 +63,17 @@ struct PipeSmem {
   static constexpr size_t kTile = sizeof(float2) * N * kW;
   static constexpr size_t kT1 = kT0 + kTile;
   static constexpr size_t kFn = kT1 + kTile;
-  static constexpr size_t kF = kFn + kTile;
-  static constexpr size_t kB = kF + kTile;
+  static constexpr size_t kB = kFn + kTile;
   static constexpr size_t kTotal = kB + sizeof(float2) * kLdB * kW;
 };
 
 // W = 16 x-lines per tile (two CTAs per SM) where the shared memory allows,
 // else 8 (n = 200, 216: three CTAs per SM).  KIND (compile time, so the
 // steady-state kernel carries none of the other cases' work):
-//   kSteady: jj >= 5 (update of iteration jj-1 >= 4: Field += Field_n,
-//            reduced in L2; source V .* Field_n)
-//   kEarly:  jj = 2, 3, 4 (first updates, the e = 3 bookkeeping, incident-
-//            field source for jj = 2)
+//   kSteady: jj >= 2 (update of iteration jj-1, source of iteration jj)
 //   kFinal:  the final pass (update of the last iteration, Field(ROI) +
 //            incident field into Fout, :646-647; no source, no forward FFT)
-enum PipeKind { kSteady = 0, kEarly = 1, kFinal = 2 };
+enum PipeKind { kSteady = 0, kFinal = 2 };
 
 template <int R2, int W, int KIND>
 __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
@@ -97,7 +93,6 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
   float2* const sT0 = reinterpret_cast<float2*>(sm + L::kT0);
   float2* const sT1 = reinterpret_cast<float2*>(sm + L::kT1);
   float2* sFn = reinterpret_cast<float2*>(sm + L::kFn);
-  float2* sF = reinterpret_cast<float2*>(sm + L::kF);
   float2* sB = reinterpret_cast<float2*>(sm + L::kB);
   const int tid = threadIdx.x;
 
@@ -138,17 +133,12 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
     mbar_arrive_expect_tx(&bar[stage], bytes);
     bulk_g2s(stage ? sT1 : sT0, a.T + tile_off(b, y0, z), bytes, &bar[stage]);
   };
-  // the steady kind only adds Field_n to Field (red_add2 in L2): no copy of
-  // Field into shared memory
-  constexpr bool kLoadF = KIND != kSteady;
   auto issue_F = [&](int t) {
     int b, y0, z, nl;
     decode(t, b, y0, z, nl);
     const uint32_t bytes = (uint32_t)(nl * N * sizeof(float2));
-    const long long o = tile_off(b, y0, z);
-    mbar_arrive_expect_tx(&bar[2], kLoadF ? 2 * bytes : bytes);
-    bulk_g2s(sFn, a.Fn + o, bytes, &bar[2]);
-    if (kLoadF) bulk_g2s(sF, a.F + o, bytes, &bar[2]);
+    mbar_arrive_expect_tx(&bar[2], bytes);
+    bulk_g2s(sFn, a.Fn + tile_off(b, y0, z), bytes, &bar[2]);
   };
   if (tid == 0) {
     issue_T(tile, 0);
@@ -159,6 +149,7 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
   const long long est = (long long)a.rx * a.ry * a.rz;
   const float2 cc = make_float2(0.f, a.c_im);
   const float2 z2 = make_float2(0.f, 0.f);
+  const bool upd = e >= 3, carry = jj >= 3;   // X in the update, in the source (see BornArgs)
 
   for (int it = 0; tile < ntiles; ++it, tile += gridDim.x) {
     const int s = it & 1;
@@ -202,13 +193,11 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
         for (int r = 0; r < kR1; ++r) Vn[r] = a.V[vb + R2 * r];
       }
     }
-    // the incident field (iteration 2's source, the final pass's Fout) is
-    // prefetched the same way; zero outside the ROI
-    constexpr bool kHasE = KIND != kSteady;
-    const bool need_e = KIND == kFinal || (KIND == kEarly && jj <= 2);
+    // the incident field (every source, the final pass's Fout) is prefetched
+    // the same way; zero outside the ROI
     auto e_load = [&](int c, int j, float2* En) {
       const int yy = c < nl ? y0 + c : y0;
-      const bool roi = need_e && (unsigned)(yy - a.ry0) < (unsigned)a.ry && (unsigned)(z - a.rz0) < (unsigned)a.rz;
+      const bool roi = (unsigned)(yy - a.ry0) < (unsigned)a.ry && (unsigned)(z - a.rz0) < (unsigned)a.rz;
       const long long base = (long long)b * est + (long long)(yy - a.ry0) * a.rx +
                              (long long)(z - a.rz0) * a.rx * a.ry - a.rx0;
 #pragma unroll
@@ -217,8 +206,8 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
         En[r] = roi && (unsigned)(x - a.rx0) < (unsigned)a.rx ? a.Einc[base + x] : z2;
       }
     };
-    float2 En[kHasE ? kR1 : 1];
-    if constexpr (kHasE) {
+    float2 En[kR1];
+    {
       int c0, j0;
       if (tid < kSlots && item(tid, c0, j0)) e_load(c0, j0, En);
     }
@@ -274,13 +263,11 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
     for (int sl = tid; sl < kSlots; sl += kThreads) {
       int c, j;
       const bool live = item(sl, c, j);
-      float2 Vv[kR1];
+      float2 Vv[kR1], Ev[kR1];
 #pragma unroll
-      for (int r = 0; r < kR1; ++r) Vv[r] = Vn[r];
-      float2 Ev[kHasE ? kR1 : 1];
-      if constexpr (kHasE) {
-#pragma unroll
-        for (int r = 0; r < kR1; ++r) Ev[r] = En[r];
+      for (int r = 0; r < kR1; ++r) {
+        Vv[r] = Vn[r];
+        Ev[r] = En[r];
       }
       {
         int cn, jn;
@@ -288,7 +275,7 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
           const int vb = v_base(cn, jn);
 #pragma unroll
           for (int r = 0; r < kR1; ++r) Vn[r] = a.V[vb + R2 * r];
-          if constexpr (kHasE) e_load(cn, jn, En);
+          e_load(cn, jn, En);
         }
       }
       if (!live) continue;
@@ -308,60 +295,26 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
         const int x = j + R2 * r;
         const float2 V = Vv[r];
         const float2 r0 = a.acyclic ? cmul(cmul(r0t[x], Ln.ry), Ln.rz) : make_float2(1.f, 0.f);
-        const bool in_roi = KIND != kSteady && Ln.roi && (unsigned)(x - a.rx0) < (unsigned)a.rx;
-        float2 Ei = z2;
-        if constexpr (kHasE) Ei = Ev[r];
         float2 P = v[r];
         if (a.acyclic) P = cmul(P, (e & 1) ? r0 : cconj(r0));
         const float m = (m0t[x] * Ln.my) * Ln.mz;
-        const float2 vP = cmul(V, P);
-        float2 ftot, fn_new;
-        if (KIND != kSteady && e <= 2) {   // Field_n = (0 + V.*PSI) .* mask
-          fn_new = cscale(vP, m);
-          // Field = 0 + Field_n after iteration 1; after iteration 2 Field
-          // keeps Field_n(1) until the e == 3 update
-          ftot = e == 1 ? fn_new : cadd(sF[c * N + x], fn_new);
-          if (KIND != kFinal && Ln.valid) {
-            a.Fn[Ln.g + x] = fn_new;
-            if (e == 1) a.F[Ln.g + x] = fn_new;
-          }
-        } else if (KIND == kSteady) {   // e >= 4: Field += Field_n (the same IEEE add, done in L2)
+        float2 xn = cmul(V, P);   // X(e) = (X(e-1) - psi + V .* PSI) .* mask
+        if (upd) {
           const float2 fo = sFn[c * N + x];
-          const float2 psi = cmul(cmul(cc, fo), V);
-          const float2 fn = cscale(cadd(csub(fo, psi), vP), m);
-          fn_new = fn;
-          ftot = z2;   // not used by this kind
-          if (Ln.valid) {
-            red_add2(a.F + Ln.g + x, fn);
-            a.Fn[Ln.g + x] = fn_new;
-          }
-        } else {
-          const float2 fo = sFn[c * N + x];
-          const float2 fp = sF[c * N + x];
-          const float2 psi = cmul(cmul(cc, fo), V);
-          const float2 fn = cscale(cadd(csub(fo, psi), vP), m);
-          if (e == 3) {  // Field = (Field_n1 + Field_n2) + Field_n3; Field_n = Field_n3 + Field_n1
-            ftot = cadd(cadd(fp, fo), fn);
-            fn_new = cadd(fn, fp);
-          } else {
-            ftot = cadd(fp, fn);
-            fn_new = fn;
-          }
-          if (KIND != kFinal && Ln.valid) {
-            a.F[Ln.g + x] = ftot;
-            a.Fn[Ln.g + x] = fn_new;
-          }
+          xn = cadd(csub(fo, cmul(cmul(cc, fo), V)), xn);
         }
-        if (KIND == kFinal) {
-          if (Ln.valid && in_roi) a.Fout[Ln.einc + x] = cadd(ftot, Ei);
+        xn = cscale(xn, m);
+        if (KIND == kFinal) {   // X(B) + X(B-1) + incident field
+          const bool in_roi = Ln.roi && (unsigned)(x - a.rx0) < (unsigned)a.rx;
+          if (e >= 2) xn = cadd(xn, sFn[c * N + x]);
+          if (Ln.valid && in_roi) a.Fout[Ln.einc + x] = cadd(xn, Ev[r]);
           continue;
         }
-        float2 src;
-        if (KIND == kEarly && jj <= 2) {  // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc) / 2 inside the ROI
-          src = in_roi ? cscale(cmul(cc, cmul(make_float2(V.x, V.y + a.eps), Ei)), 0.5f) : z2;
-        } else {        // (1i/eps) .* Field_n .* V
-          src = cmul(cmul(cc, fn_new), V);
-        }
+        if (Ln.valid) a.Fn[Ln.g + x] = xn;
+        // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc / 2 + V .* X); E_inc = 0 outside the ROI
+        float2 q = cscale(cmul(make_float2(V.x, V.y + a.eps), Ev[r]), 0.5f);
+        if (carry) q = cadd(q, cmul(xn, V));
+        float2 src = cmul(cc, q);
         if (a.acyclic) src = cmul(src, (jj & 1) ? cconj(r0) : r0);
         v[r] = Ln.valid ? src : z2;
       }
@@ -467,13 +420,11 @@ bool born_x_pipe_supported(const BornArgs& a, const DevFft& fx) {
 cudaError_t launch_born_x_pipe(const BornArgs& a, int mode, int jj, const DevFft& fx, int* fault,
                                cudaStream_t s) {
   if (jj < 2 || (mode != kBornMid && mode != kBornLast)) return cudaErrorInvalidValue;
-  const int kind = mode == kBornLast ? kFinal : (jj <= 4 ? kEarly : kSteady);
   switch (a.px / kR1) {
 #define ODT_PIPE_CASE(R)                                                     \
   case R:                                                                    \
-    return kind == kFinal   ? launch_r2<R, kFinal>(a, jj, fx, fault, s)      \
-           : kind == kEarly ? launch_r2<R, kEarly>(a, jj, fx, fault, s)      \
-                            : launch_r2<R, kSteady>(a, jj, fx, fault, s);
+    return mode == kBornLast ? launch_r2<R, kFinal>(a, jj, fx, fault, s)     \
+                             : launch_r2<R, kSteady>(a, jj, fx, fault, s);
     ODT_PIPE_CASE(11)
     ODT_PIPE_CASE(15)
     ODT_PIPE_CASE(19)

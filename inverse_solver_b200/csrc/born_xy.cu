@@ -96,7 +96,8 @@ struct XYSmem {
 };
 
 // KIND: which Born iterations a launch serves (compile time, so the steady
-// kernel carries none of the other cases' work)
+// kernel carries none of the other cases' work); the early kind exists for
+// the 16-bit storage's term-by-term series only (its iterations 2-4)
 enum XYKind { kXYSteady = 0, kXYEarly = 1, kXYFinal = 2, kXYFirst = 3 };
 
 // (i c) * v for real c: (-c v.y, c v.x), two products (a complex product
@@ -148,14 +149,18 @@ __global__ void __launch_bounds__(32 * R, 1)
   const int e = jj - 1;                     // iteration whose update completes here
   const long long plane_n = (long long)N * N;
   const long long est = (long long)a.rx * a.ry * a.rz;
-  // Field_n / Field are read by the update from iteration 3 on (and Field by
-  // the final pass of a 2-iteration series); the incident field by the
-  // source of iteration 1 and 2 and by the final pass
-  const bool need_fn = kInv && e >= 3;
-  // the steady kind only adds Field_n to Field, with a reduction in L2
-  // (red.global.add: no load of Field on the way)
-  const bool need_f = KIND != kXYSteady && kInv && (e >= 3 || (KIND == kXYFinal && e == 2));
-  const bool need_e = KIND == kXYFinal || ((KIND == kXYFirst || KIND == kXYEarly) && jj <= 2);
+  // complex64 storage (the nested form, see BornArgs): X(e-1) is part of the
+  // update from iteration 3 on and of the result from 2 on, the incident
+  // field part of every source.  16-bit storage (term by term): Field_n and
+  // Field are read by the update from iteration 3 on (and Field by the final
+  // pass of a 2-iteration series), the incident field by the source of
+  // iterations 1 and 2 and by the final pass; its steady kind only adds
+  // Field_n to Field, with a reduction in L2 (red.global.add: no load)
+  const bool upd = e >= 3;
+  const bool carry = jj >= 3;   // the source of iterations 1 and 2 has no X
+  const bool need_fn = kInv && (upd || (ST == 0 && KIND == kXYFinal && e == 2));
+  const bool need_f = ST == 1 && KIND != kXYSteady && kInv && (upd || (KIND == kXYFinal && e == 2));
+  const bool need_e = ST == 0 || KIND == kXYFinal || ((KIND == kXYFirst || KIND == kXYEarly) && jj <= 2);
 
   // ---- 1: y-F3^-1 (R-point over k2 at rows R k1 + k2) and twiddles of item
   // i = (x, k1) of the plane at g0, from T into the plane buffer
@@ -244,7 +249,7 @@ __global__ void __launch_bounds__(32 * R, 1)
       // ramp(x) ry rz: per element one product with the x factor)
       const float myz = myt[y] * mz;
       const float2 ryz = a.acyclic ? cmul(ryt[y], rz) : one;
-      float2 V[8], Fo[8], Fp[8], Ei[8];
+      float2 V[8], Fo[8], Fp[ST == 1 ? 8 : 1], Ei[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const int x = R * r + n2;
@@ -255,7 +260,7 @@ __global__ void __launch_bounds__(32 * R, 1)
         } else {
           Fo[r] = need_fn ? b16_decode(a.Fn16[gy + x], a.Fe[fe + r * R * R]) : z2;
         }
-        Fp[r] = need_f ? a.F[gy + x] : z2;
+        if constexpr (ST == 1) Fp[r] = need_f ? a.F[gy + x] : z2;
         Ei[r] = (need_e && in_roi) ? a.Einc[ebase + x] : z2;
       }
       // Field_n of element (x, y) of the item's r-th value (the 8 lanes of a
@@ -288,7 +293,12 @@ __global__ void __launch_bounds__(32 * R, 1)
           if (a.acyclic) P = cmul(P, (e & 1) ? r0 : cconj(r0));
           const float m = mxt[x] * myz;
           const float2 vP = cmul(Vr, P);
-          if (KIND != kXYSteady && e <= 2) {   // Field_n = (0 + V .* PSI) .* mask
+          if constexpr (ST == 0) {   // X(e) = (X(e-1) - psi + V .* PSI) .* mask
+            fn_new = upd ? cadd(csub(Fo[r], cmul(mul_i(a.c_im, Fo[r]), Vr)), vP) : vP;
+            fn_new = cscale(fn_new, m);
+            if (KIND == kXYFinal) ftot = cadd(fn_new, Fo[r]);
+            else store_fn(r, x, fn_new);
+          } else if (KIND != kXYSteady && e <= 2) {   // Field_n = (0 + V .* PSI) .* mask
             fn_new = cscale(vP, m);
             // Field = 0 + Field_n after iteration 1; after iteration 2 Field
             // keeps Field_n(1) until the e == 3 update
@@ -325,7 +335,11 @@ __global__ void __launch_bounds__(32 * R, 1)
           if (in_roi) a.Fout[ebase + x] = cadd(ftot, Ei[r]);
         } else {
           float2 src;
-          if (jj <= 2) {  // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc) / 2 inside the ROI
+          if constexpr (ST == 0) {   // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc / 2 + V .* X)
+            float2 q = cscale(cmul(make_float2(Vr.x, Vr.y + a.eps), Ei[r]), 0.5f);   // E_inc = 0 outside the ROI
+            if (KIND == kXYSteady && carry) q = cadd(q, cmul(fn_new, Vr));
+            src = mul_i(a.c_im, q);
+          } else if (jj <= 2) {  // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc) / 2 inside the ROI
             src = in_roi ? cscale(mul_i(a.c_im, cmul(make_float2(Vr.x, Vr.y + a.eps), Ei[r])), 0.5f) : z2;
           } else {        // (1i/eps) .* Field_n .* V
             src = cmul(mul_i(a.c_im, fn_new), Vr);
@@ -435,7 +449,9 @@ template <int R, int ST>
 cudaError_t launch_kind_st(const BornArgs& a, int kind, int jj, const float2* tw, cudaStream_t s) {
   switch (kind) {
     case kXYSteady: return launch_r<R, kXYSteady, ST>(a, jj, tw, s);
-    case kXYEarly: return launch_r<R, kXYEarly, ST>(a, jj, tw, s);
+    case kXYEarly:
+      if constexpr (ST == 1) return launch_r<R, kXYEarly, ST>(a, jj, tw, s);
+      return cudaErrorInvalidValue;
     case kXYFinal: return launch_r<R, kXYFinal, ST>(a, jj, tw, s);
     default: return launch_r<R, kXYFirst, ST>(a, jj, tw, s);
   }
@@ -474,8 +490,8 @@ cudaError_t launch_born_xy(const BornArgs& a, int mode, int jj, const DevFft& fx
   int kind;
   if (mode == kBornFirst) kind = kXYFirst;
   else if (mode == kBornLast) kind = kXYFinal;
-  else kind = jj <= 4 ? kXYEarly : kXYSteady;   // steady: e = jj - 1 >= 4 (Field += Field_n only)
-  if ((mode == kBornFirst) != (jj == 1)) return cudaErrorInvalidValue;
+  else kind = a.storage && jj <= 4 ? kXYEarly : kXYSteady;   // 16-bit steady: e >= 4 (Field += Field_n only)
+  if (mode == kBornFirst ? jj > (a.storage ? 1 : 2) : jj < 2) return cudaErrorInvalidValue;
   switch (a.px / 8) {
     case 11: return launch_kind<11>(a, kind, jj, fx.tw, s);
     case 12: return launch_kind<12>(a, kind, jj, fx.tw, s);

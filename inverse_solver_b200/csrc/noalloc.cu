@@ -168,8 +168,9 @@ extern "C" odt_status odt_born_series_noalloc(const odt_noalloc_born_args* a) {
   b.Fout = reinterpret_cast<float2*>(a->fout);
   b.wait_limit = kWaitLimitCycles;
   const int B = a->bornmax;
-  for (int jj = 1; jj <= B && e == cudaSuccess; ++jj) {
-    if ((e = launch_born_x(b, jj == 1 ? kBornFirst : kBornMid, jj, f[0], s)) != cudaSuccess) break;
+  const int j0 = B >= 3 ? 2 : 1;   // the nested series starts with iteration 2 (see BornArgs)
+  for (int jj = j0; jj <= B && e == cudaSuccess; ++jj) {
+    if ((e = launch_born_x(b, jj == j0 ? kBornFirst : kBornMid, jj, f[0], s)) != cudaSuccess) break;
     if ((e = launch_fft_cols(b.T, b.T, b.px, (long long)b.pz, 0, 0, 1.0f, false, f[1], s)) != cudaSuccess) break;
     if ((e = launch_born_z(b, jj, f[2], s)) != cudaSuccess) break;
     e = launch_fft_cols(b.T, b.T, b.px, (long long)b.pz, 0, 0, 1.0f, true, f[1], s);

@@ -89,10 +89,10 @@ struct DeviceGuard {
 const char* const kKindNames[] = {"born_x", "born_y", "born_z", "io_fft", "io_elementwise",
                                   "born_x_pipe", "born_y_pipe", "born_z_pipe", "born_x_pipe_edge",
                                   "born_xy", "born_xy_edge"};
-// born_x_pipe_edge: the pipelined x-pass of iterations 2, 3 and of the final
-// pass (incident-field source / output), timed apart from the steady state;
-// born_xy / born_xy_edge: the fused xy-pass, steady (iterations 4..Bornmax)
-// and edge (iterations 1-3 and the final pass)
+// born_x_pipe_edge: the pipelined x-pass's final pass (output), timed apart
+// from the steady state; born_xy / born_xy_edge: the fused xy-pass, steady
+// and edge (the first source and the final pass; with 16-bit storage also
+// iterations 2-4)
 enum Kind { kKBornX = 0, kKBornY, kKBornZ, kKIoFft, kKIoElem, kKBornXPipe, kKBornYPipe, kKBornZPipe,
             kKBornXPipeEdge, kKBornXY, kKBornXYEdge, kNumKinds };
 
@@ -570,6 +570,10 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   a.Fout = fout;
   a.wait_limit = H.wait_limit;
   const int B = P.pp.bornmax;
+  // the nested form of the series starts with iteration 2 (see BornArgs; a
+  // series of one or two iterations with 1); 16-bit storage and RI tensors
+  // go term by term
+  const int j0 = B >= 3 && !ten && H.storage != ODT_STORAGE_B16 ? 2 : 1;
   if (H.any_loop()) {
     // unfused loop with Bluestein transforms along the uncovered axes
     if (ten || vec) raise(ODT_ERR_UNSUPPORTED, "RI tensors and dyadic solves need padded lengths whose prime "
@@ -594,10 +598,10 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
       if (inv) { az(); ay(); ax(); } else { ax(); ay(); az(); }
       H.mark_end(s);
     };
-    for (int jj = 1; jj <= B; ++jj) {
-      if (jj >= 2) fft3(true);
+    for (int jj = j0; jj <= B; ++jj) {
+      if (jj > j0) fft3(true);
       H.mark_begin(kKBornX, s);
-      ODT_CUDA(launch_born_point(a, jj == 1 ? kBornFirst : kBornMid, jj, s));
+      ODT_CUDA(launch_born_point(a, jj == j0 ? kBornFirst : kBornMid, jj, s));
       H.mark_end(s);
       fft3(false);
       H.mark_begin(kKBornZ, s);
@@ -643,9 +647,9 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     a.T = nullptr;
     a.Fn = nullptr;
   }
-  for (int jj = 1; fused_xy && jj <= B; ++jj) {
-    H.mark_begin(jj <= 4 ? kKBornXYEdge : kKBornXY, s);
-    ODT_CUDA(launch_born_xy(a, jj == 1 ? kBornFirst : kBornMid, jj, H.fx, s));
+  for (int jj = j0; fused_xy && jj <= B; ++jj) {
+    H.mark_begin(jj == j0 || (a.storage && jj <= 4) ? kKBornXYEdge : kKBornXY, s);
+    ODT_CUDA(launch_born_xy(a, jj == j0 ? kBornFirst : kBornMid, jj, H.fx, s));
     H.mark_end(s);
     H.mark_begin(pipe_z ? kKBornZPipe : kKBornZ, s);
     if (pipe_z)
@@ -659,18 +663,18 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     ODT_CUDA(launch_born_xy(a, kBornLast, B + 1, H.fx, s));
     H.mark_end(s);
   }
-  for (int jj = 1; !any && !fused_xy && jj <= B; ++jj) {
+  for (int jj = j0; !any && !fused_xy && jj <= B; ++jj) {
     if (ten) {  // plain x-FFTs around the component-coupling pointwise kernel
       H.mark_begin(kKBornX, s);
       if (jj >= 2) ODT_CUDA(launch_fft_lines(a.T, a.T, xlines, 0, 0, 1.0f, true, H.fx, s));
       ODT_CUDA(launch_born_tensor_point(a, P.V9, jj == 1 ? kBornFirst : kBornMid, jj, s));
       ODT_CUDA(launch_fft_lines(a.T, a.T, xlines, 0, 0, 1.0f, false, H.fx, s));
-    } else if (pipe_x && jj >= 2) {
-      H.mark_begin(jj <= 4 ? kKBornXPipeEdge : kKBornXPipe, s);
+    } else if (pipe_x && jj > j0) {
+      H.mark_begin(kKBornXPipe, s);
       ODT_CUDA(launch_born_x_pipe(a, kBornMid, jj, H.fx, H.d_fault, s));
     } else {
       H.mark_begin(kKBornX, s);
-      ODT_CUDA(launch_born_x(a, jj == 1 ? kBornFirst : kBornMid, jj, H.fx, s));
+      ODT_CUDA(launch_born_x(a, jj == j0 ? kBornFirst : kBornMid, jj, H.fx, s));
     }
     H.mark_end(s);
     H.mark_begin(pipe_y ? kKBornYPipe : kKBornY, s);

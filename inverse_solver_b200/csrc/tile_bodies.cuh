@@ -4,11 +4,12 @@
 //
 //   born_x_body : x-pass of Born iteration jj -- inverse x-FFT of the
 //                 spectral array, completion of the update of iteration jj-1
-//                 (FORWARD_SOLVER_CONVERGENT_BORN.m:616-642), the source term
-//                 of iteration jj (:588-605) times the phase ramp, forward
-//                 x-FFT.  Modes: First (jj = 1: source only), Mid, Last
-//                 (update of the final iteration, writes Field(ROI) + incident
-//                 field, :646-647).
+//                 (FORWARD_SOLVER_CONVERGENT_BORN.m:616-642, in the nested
+//                 form described at BornArgs), the source term of iteration
+//                 jj (:588-605) times the phase ramp, forward x-FFT.  Modes:
+//                 First (jj = 1 or 2: source only), Mid, Last (update of the
+//                 final iteration, writes Field(ROI) + incident field,
+//                 :646-647).
 //   born_z_body : forward z-FFT, Green's multiply G(k -/+ dk/4) with the
 //                 1/N of ifftn folded in (:608-615), inverse z-FFT.
 //   fft_lines_body / fft_cols_body : plain batched FFTs (y-pass of the Born
@@ -64,77 +65,44 @@ struct BornXOp {
     }
     const int e = jj - 1;  // iteration whose update completes here
     const bool upd = MODE != kBornFirst && e >= 1;
-    const bool need_fn = upd && e >= 3;
-    const bool need_f = upd && (e >= 3 || (MODE == kBornLast && e == 2));
-    const bool need_einc = MODE == kBornLast || jj <= 2;
+    // X(e-1): part of the update from iteration 3 on, of the result from 2 on
+    const bool need_x = upd && (e >= 3 || (MODE == kBornLast && e == 2));
     const float2 z2 = make_float2(0.f, 0.f);
-    float2 Vv[R], Fo[R], Fp[R], Ei[R];
+    float2 Vv[R], Xo[R], Ei[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int x = j + r * nb;
-      const long long gi = L.g + x;
       const bool in_roi = L.roi && (unsigned)(x - A.rx0) < (unsigned)A.rx;
       Vv[r] = A.V[L.v + x];
-      Fo[r] = need_fn ? A.Fn[gi] : z2;
-      Fp[r] = need_f ? A.F[gi] : z2;
-      Ei[r] = (need_einc && in_roi) ? A.Einc[L.einc + x] : z2;
+      Xo[r] = need_x ? A.Fn[L.g + x] : z2;
+      Ei[r] = in_roi ? A.Einc[L.einc + x] : z2;
     }
     const float2 cc = make_float2(0.f, A.c_im);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int x = j + r * nb;
-      const long long gi = L.g + x;
       const float2 V = Vv[r];
       const float2 r0 = A.acyclic ? cmul(cmul(A.ramp[0][x], L.ry), L.rz) : make_float2(1.f, 0.f);
       const bool in_roi = L.roi && (unsigned)(x - A.rx0) < (unsigned)A.rx;
-      float2 fn_new = z2;
-      float2 ftot = z2;
+      float2 xn = z2;
       if (upd) {
         // PSI = ifftn(...) .* conj(phase_ramp_e), phase_ramp_e = conj(r0) for odd e
         float2 P = v[r];
         if (A.acyclic) P = cmul(P, (e & 1) ? r0 : cconj(r0));
         const float m = (A.mask[0][x] * L.my) * L.mz;
-        const float2 vP = cmul(V, P);
-        if (e <= 2) {
-          fn_new = cscale(vP, m);  // (0 + V.*PSI) .* mask
-          if (MODE == kBornMid) {
-            A.Fn[gi] = fn_new;
-            if (e == 1) A.F[gi] = fn_new;  // Field = 0 + Field_n
-            // e == 2: Field keeps Field_n(1) until the e == 3 update
-          } else {
-            ftot = (e == 1) ? fn_new : cadd(Fp[r], fn_new);
-          }
-        } else {
-          const float2 fo = Fo[r];
-          const float2 psi = cmul(cmul(cc, fo), V);
-          const float2 fn = cscale(cadd(csub(fo, psi), vP), m);
-          const float2 fp = Fp[r];
-          if (e == 3) {  // Field = (Field_n1 + Field_n2) + Field_n3; Field_n = Field_n3 + Field_n1
-            ftot = cadd(cadd(fp, fo), fn);
-            fn_new = cadd(fn, fp);
-          } else {
-            ftot = cadd(fp, fn);
-            fn_new = fn;
-          }
-          if (MODE == kBornMid) {
-            A.F[gi] = ftot;
-            A.Fn[gi] = fn_new;
-          }
-        }
+        xn = cmul(V, P);
+        if (e >= 3) xn = cadd(csub(Xo[r], cmul(cmul(cc, Xo[r]), V)), xn);
+        xn = cscale(xn, m);
+        if (MODE == kBornMid) A.Fn[L.g + x] = xn;
       }
-      if (MODE == kBornLast) {
-        if (in_roi) A.Fout[L.einc + x] = cadd(ftot, Ei[r]);
+      if (MODE == kBornLast) {   // X(B) + X(B-1) + incident field
+        if (in_roi) A.Fout[L.einc + x] = cadd(cadd(xn, Xo[r]), Ei[r]);
         continue;
       }
-      float2 psi = z2;
-      if (jj <= 2) {  // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc) / 2 inside the ROI
-        if (in_roi) {
-          const float2 sv = cmul(make_float2(V.x, V.y + A.eps), Ei[r]);
-          psi = cscale(cmul(cc, sv), 0.5f);
-        }
-      } else {  // (1i/eps) .* Field_n .* V
-        psi = cmul(cmul(cc, fn_new), V);
-      }
+      // (1i/eps) .* ((V(ROI) + 1i*eps) .* E_inc / 2 + V .* X)
+      float2 w = in_roi ? cscale(cmul(make_float2(V.x, V.y + A.eps), Ei[r]), 0.5f) : z2;
+      if (jj >= 3 && MODE == kBornMid) w = cadd(w, cmul(xn, V));
+      float2 psi = cmul(cc, w);
       if (A.acyclic) psi = cmul(psi, (jj & 1) ? cconj(r0) : r0);
       v[r] = psi;
     }
