@@ -14,7 +14,8 @@
 // double on the host and rounded once to float (the accuracy of the table
 // bounds the accuracy of the transform; nothing here calls sin/cos).
 //
-// Radices: 2, 4, 8 (closed-form butterflies) and any odd R <= 31 through the
+// Radices: 2, 4, 8 (closed-form butterflies), composite ones from two smaller
+// butterflies, and odd primes <= 31 through the
 // symmetric real-coefficient DFT (pairs v[m], v[R-m] so that an odd R-point
 // DFT costs (R-1)^2 real multiply-adds instead of R^2 complex products).
 //
@@ -238,7 +239,7 @@ struct Butterfly<12, INV> {
   }
 };
 
-// Odd R: X[k] = v0 + sum_m a_m cos(2 pi m k / R) -/+ i sum_m b_m sin(2 pi m k / R)
+// Odd prime R: X[k] = v0 + sum_m a_m cos(2 pi m k / R) -/+ i sum_m b_m sin(2 pi m k / R)
 // with a_m = v[m] + v[R-m], b_m = v[m] - v[R-m]; the cosines and sines are
 // read from the transform's table at multiples of n / R.
 template <int R, bool INV>
@@ -249,7 +250,7 @@ struct OddButterfly {
     (void)tw;
     (void)n;
     float cs[H + 1], sn[H + 1];
-    cs[0] = 1.f;  // m*k can be a multiple of R when R is composite (9, 15, ...)
+    cs[0] = 1.f;
     sn[0] = 0.f;
 #pragma unroll
     for (int t = 1; t <= H; ++t) {
@@ -340,43 +341,42 @@ struct CompositeButterfly {
 ODT_ODD_BUTTERFLY(3)
 ODT_ODD_BUTTERFLY(5)
 ODT_ODD_BUTTERFLY(7)
-ODT_ODD_BUTTERFLY(9)
 ODT_ODD_BUTTERFLY(11)
 ODT_ODD_BUTTERFLY(13)
-ODT_ODD_BUTTERFLY(15)
 ODT_ODD_BUTTERFLY(17)
 ODT_ODD_BUTTERFLY(19)
 ODT_ODD_BUTTERFLY(23)
-ODT_ODD_BUTTERFLY(25)
-ODT_ODD_BUTTERFLY(27)
 ODT_ODD_BUTTERFLY(29)
 ODT_ODD_BUTTERFLY(31)
 #undef ODT_ODD_BUTTERFLY
 
-template <bool INV>
-struct Butterfly<35, INV> {
-  ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<5, 7, INV>::run(v, tw, n); }
-};
-
-// even radices of the fused xy-pass and the pipelined z-pass (axes of
-// 8 R = 112, 128, 144, 160 points): 14 = 2 x 7, 16 = 4 x 4, 18 = 2 x 9,
-// 20 = 4 x 5
-template <bool INV>
-struct Butterfly<14, INV> {
-  ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<2, 7, INV>::run(v, tw, n); }
-};
-template <bool INV>
-struct Butterfly<16, INV> {
-  ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<4, 4, INV>::run(v, tw, n); }
-};
-template <bool INV>
-struct Butterfly<18, INV> {
-  ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<2, 9, INV>::run(v, tw, n); }
-};
-template <bool INV>
-struct Butterfly<20, INV> {
-  ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<4, 5, INV>::run(v, tw, n); }
-};
+// Composite radices.  The symmetric DFT costs (R - 1)^2 real multiply-adds,
+// the two-factor form A (B - 1)^2 + B (A - 1)^2 and four operations per inner
+// twiddle: 676 against about 300 for 27 = 3 x 9, 576 against 224 for 25,
+// 196 against 100 for 15, 64 against 40 for 9.
+#define ODT_COMPOSITE_BUTTERFLY(A, B)                                                                      \
+  template <bool INV>                                                                                     \
+  struct Butterfly<A * B, INV> {                                                                          \
+    ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<A, B, INV>::run(v, tw, n); } \
+  };
+ODT_COMPOSITE_BUTTERFLY(2, 3)
+ODT_COMPOSITE_BUTTERFLY(3, 3)
+ODT_COMPOSITE_BUTTERFLY(2, 5)
+ODT_COMPOSITE_BUTTERFLY(2, 7)
+ODT_COMPOSITE_BUTTERFLY(3, 5)
+ODT_COMPOSITE_BUTTERFLY(4, 4)
+ODT_COMPOSITE_BUTTERFLY(2, 9)
+ODT_COMPOSITE_BUTTERFLY(4, 5)
+ODT_COMPOSITE_BUTTERFLY(3, 7)
+ODT_COMPOSITE_BUTTERFLY(2, 11)
+ODT_COMPOSITE_BUTTERFLY(3, 8)
+ODT_COMPOSITE_BUTTERFLY(5, 5)
+ODT_COMPOSITE_BUTTERFLY(2, 13)
+ODT_COMPOSITE_BUTTERFLY(3, 9)
+ODT_COMPOSITE_BUTTERFLY(4, 7)
+ODT_COMPOSITE_BUTTERFLY(5, 6)
+ODT_COMPOSITE_BUTTERFLY(5, 7)
+#undef ODT_COMPOSITE_BUTTERFLY
 
 // ------------------------------------------------------------------ one pass
 // Stockham radix-R pass over a tile of W pencils (W a power of two, lgW its
