@@ -1,24 +1,23 @@
-// Pipelined column passes of the Born iteration for lengths n = 8 * R2 (R2
-// odd): the y-FFTs (forward / inverse, in place on T) and the z-pass
-// (forward z-FFT, Green's multiply G(k -/+ dk/4) / N, inverse z-FFT;
+// Pipelined column passes of the Born iteration for lengths n = 8 * R2: the
+// y-FFTs (forward / inverse, in place on T) and the z-pass of the 16-bit block
+// storage (forward z-FFT, Green's multiply G(k -/+ dk/4) / N, inverse z-FFT;
 // FORWARD_SOLVER_CONVERGENT_BORN.m:606-615) -- the same transforms as
 // fft_cols_body / born_z_body, restructured like the pipelined x-pass:
 //
-//   * persistent CTAs (as many per SM as shared memory and registers allow:
-//     three for the y-FFTs, five for the z-pass at n <= 152) walk tiles of
-//     16 adjacent columns;
-//   * a tile (16 columns x n rows, each row a 128-byte segment at a stride of
-//     px or px*py elements) arrives in shared memory through one tiled TMA
-//     copy (cp.async.bulk.tensor, 3D map for y, 4D for z) on an mbarrier,
-//     while the CTA computes the previous tile from the other stage;
+//   * persistent CTAs (as many per SM as shared memory and registers allow)
+//     walk tiles of 16 adjacent columns;
+//   * a tile (16 columns x n rows, each row a 128-byte segment (64 bytes in
+//     16-bit storage) at a stride of px or px*py elements) arrives in shared
+//     memory through one tiled TMA copy (cp.async.bulk.tensor, 3D map for y,
+//     4D for z) on an mbarrier, while the CTA computes the previous tile from
+//     the other stage;
 //   * y-FFTs: radix-R2 pass in place in the landing buffer (one butterfly
 //     per thread held in registers across a barrier), then radix-8 with
 //     twiddles straight to global memory;
 //   * z-pass: with z = R2 n1 + n2 and kz = k1 + 8 k2, an 8-point DFT over n1
 //     with twiddles, then per (column, k1) the R2-point DFT, the Green's
 //     multiply at kz and the inverse R2-point DFT in registers, then the
-//     inverse 8-point DFT to global memory; every step writes the rows it
-//     read, so the landing buffer is the only buffer.
+//     inverse 8-point DFT to global memory, in place on the decoded tile.
 //
 // Layout in shared memory: [row][column], 16 columns = 128 bytes per row; the
 // column index is the fastest thread index, so every access of a half-warp
@@ -45,7 +44,7 @@ constexpr int kThreads = kW * kR1;   // y-FFTs: one radix-R2 butterfly per threa
 // rounds for R2 <= 19 instead of three; step B uses the first 128
 constexpr int kThreadsZ = 160;
 template <int KIND>
-__host__ __device__ constexpr int threads_of() { return KIND >= 2 ? kThreadsZ : kThreads; }
+__host__ __device__ constexpr int threads_of() { return KIND == 3 ? kThreadsZ : kThreads; }
 
 constexpr size_t a16(size_t b) { return (b + 15) & ~(size_t)15; }
 constexpr size_t a1k(size_t b) { return (b + 1023) & ~(size_t)1023; }
@@ -62,8 +61,7 @@ struct ColSmem {
   static constexpr size_t kS0 = a1k(kGxy + a16(sizeof(float) * kW));
   static constexpr size_t kS1 = kS0 + kTile;
   static constexpr size_t kB = kS1 + kTile;
-  static constexpr size_t kTotalY = kB;                             // both kinds: two stages only
-  static constexpr size_t kTotalZ = kB;
+  static constexpr size_t kTotalY = kB;                             // two stages only
   // z-pass on 16-bit block floating-point storage: two landing stages of
   // int16 (re, im) pairs, one complex64 work tile, the tile's exponents
   static constexpr size_t kTile16 = sizeof(short2) * N * kW;
@@ -101,21 +99,21 @@ __device__ __forceinline__ float rcp_approx(float x) {
 }
 #endif
 
-// KIND 0: forward y-FFT, 1: inverse y-FFT, 2: z-pass with Green's multiply,
-// 3: the z-pass on 16-bit block floating-point storage (a.T16 / a.Te: the
-// tile lands as int16 pairs, is decoded into a complex64 work tile and the
-// result is encoded again with one exponent per 8 columns of a row).
+// KIND 0: forward y-FFT, 1: inverse y-FFT, 3: the z-pass on 16-bit block
+// floating-point storage (a.T16 / a.Te: the tile lands as int16 pairs, is
+// decoded into a complex64 work tile and the result is encoded again with one
+// exponent per 8 columns of a row; complex64 storage has z_pass.cu).
 // Tile t -> (x-tile fastest, then the outer index o): y-pass o = z + pz*b
 // (3D map {px, py, pz*nb}), z-pass o = y + py*b (4D map {px, py, pz, nb}).
 template <int R2, int KIND>
-__global__ void __launch_bounds__(threads_of<KIND>(), KIND >= 2 ? (R2 <= 19 ? 5 : 4) : 3)
+__global__ void __launch_bounds__(threads_of<KIND>(), KIND == 3 ? (R2 <= 19 ? 5 : 4) : 3)
     cols_pipe_kernel(const __grid_constant__ CUtensorMap map, const BornArgs a, const int jj,
                      const float2* __restrict__ twg, const int nxt, const int ntiles,
                      int* __restrict__ fault) {
 #if defined(__CUDA_ARCH__)
   constexpr int N = kR1 * R2;
-  constexpr bool kZ = KIND >= 2;
-  constexpr bool k16 = KIND == 3;
+  constexpr bool kZ = KIND == 3;
+  constexpr bool k16 = kZ;
   constexpr int kT = threads_of<KIND>();
   // y-columns longer than a TMA box dimension (256) arrive as two halves
   constexpr bool kSplitY = !kZ && N > 256;
@@ -158,8 +156,7 @@ __global__ void __launch_bounds__(threads_of<KIND>(), KIND >= 2 ? (R2 <= 19 ? 5 
     const int xt = t % nxt, o = t / nxt;
     mbar_arrive_expect_tx(&bar[stage], kBytes);
     float2* dst = stage ? s1 : s0;
-    if (k16) tma_load_4d(dst, &map, kW * xt, o % a.py, 0, o / a.py, &bar[stage]);
-    else if (kZ) tma_load_4d(dst, &map, 2 * kW * xt, o % a.py, 0, o / a.py, &bar[stage]);
+    if (kZ) tma_load_4d(dst, &map, kW * xt, o % a.py, 0, o / a.py, &bar[stage]);
     else if (kSplitY) {
       tma_load_3d(dst, &map, 2 * kW * xt, 0, o, &bar[stage]);
       tma_load_3d(dst + (N / 2) * kW, &map, 2 * kW * xt, N / 2, o, &bar[stage]);
@@ -247,20 +244,15 @@ __global__ void __launch_bounds__(threads_of<KIND>(), KIND >= 2 ? (R2 <= 19 ? 5 
       //   B  R2-point DFT over n2 at rows R2 k1 + n2 (kz = k1 + 8 k2), Green's
       //      multiply, inverse R2-point DFT, times conj W_N^(n2 k1)
       //   C  inverse 8-point DFT over k1 -> rows R2 n1 + n2 of T
-      float2* const Wt = k16 ? w16 : S;   // the tile the steps work on
+      float2* const Wt = w16;   // the tile the steps work on
       for (int idx = tid; idx < kW * R2; idx += kT) {
         const int n2 = idx >> 4;  // column c is idx & 15 == tid & 15
         float2 v[kR1];
-        if constexpr (k16) {
-          const short2* S16 = reinterpret_cast<const short2*>(S);
+        const short2* S16 = reinterpret_cast<const short2*>(S);
 #pragma unroll
-          for (int r = 0; r < kR1; ++r) {
-            const int row = R2 * r + n2;
-            v[r] = b16_decode(S16[row * kW + c], exs[2 * row + (c >> 3)]);
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < kR1; ++r) v[r] = S[(R2 * r + n2) * kW + c];
+        for (int r = 0; r < kR1; ++r) {
+          const int row = R2 * r + n2;
+          v[r] = b16_decode(S16[row * kW + c], exs[2 * row + (c >> 3)]);
         }
         Butterfly<kR1, false>::run(v, tw, N);
 #pragma unroll
@@ -297,22 +289,17 @@ __global__ void __launch_bounds__(threads_of<KIND>(), KIND >= 2 ? (R2 <= 19 ? 5 
 #pragma unroll
         for (int r = 0; r < kR1; ++r) v[r] = Wt[(R2 * r + n2) * kW + c];
         Butterfly<kR1, true>::run(v, tw, N);
-        if constexpr (k16) {   // lanes 8j .. 8j+7 hold columns 8h .. 8h+7 of the same rows
-          const unsigned mask = __activemask();
-          short2* out = a.T16 + gbase + c;
+        // lanes 8j .. 8j+7 hold columns 8h .. 8h+7 of the same rows
+        const unsigned mask = __activemask();
+        short2* out = a.T16 + gbase + c;
 #pragma unroll
-          for (int r = 0; r < kR1; ++r) {
-            const int ex = b16_group_exponent(v[r], mask);
-            const long long off = (long long)(R2 * r + n2) * rstride;
-            if (c < ncol) {
-              out[off] = b16_encode(v[r], ex);
-              if ((c & 7) == 0) a.Te[(gbase + c + off) >> 3] = (signed char)ex;
-            }
+        for (int r = 0; r < kR1; ++r) {
+          const int ex = b16_group_exponent(v[r], mask);
+          const long long off = (long long)(R2 * r + n2) * rstride;
+          if (c < ncol) {
+            out[off] = b16_encode(v[r], ex);
+            if ((c & 7) == 0) a.Te[(gbase + c + off) >> 3] = (signed char)ex;
           }
-        } else if (c < ncol) {
-          float2* out = a.T + gbase + c;
-#pragma unroll
-          for (int r = 0; r < kR1; ++r) out[(R2 * r + n2) * rstride] = v[r];
         }
       }
       if constexpr (k16) {
@@ -381,7 +368,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 // {2*px, py, pz, nb} (z-pass); box 32 floats = 16 complex columns.  With
 // 16-bit storage (b16) the map covers T16 viewed as 32-bit (re, im) int16
 // pairs: dims {px, py, pz, nb}, box 16 columns (64 bytes).
-bool make_map(const BornArgs& a, bool zpass, CUtensorMap* m, bool b16 = false) {
+bool make_map(const BornArgs& a, CUtensorMap* m, bool b16) {
   auto enc = encoder();
   if (!enc) return false;
   const cuuint64_t px2 = 2ull * a.px;
@@ -397,7 +384,7 @@ bool make_map(const BornArgs& a, bool zpass, CUtensorMap* m, bool b16 = false) {
     r = enc(m, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, a.T16, dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  } else if (!zpass) {
+  } else {
     const cuuint64_t dims[3] = {px2, (cuuint64_t)a.py, (cuuint64_t)a.pz * a.nbatch};
     const cuuint64_t strides[2] = {rowb, planeb};
     // a box dimension holds at most 256 elements: longer columns (280) land
@@ -407,13 +394,6 @@ bool make_map(const BornArgs& a, bool zpass, CUtensorMap* m, bool b16 = false) {
     r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, a.T, dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  } else {
-    const cuuint64_t dims[4] = {px2, (cuuint64_t)a.py, (cuuint64_t)a.pz, (cuuint64_t)a.nbatch};
-    const cuuint64_t strides[3] = {rowb, planeb, planeb * a.pz};
-    const cuuint32_t box[4] = {2 * kW, 1, (cuuint32_t)a.pz, 1};
-    r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.T, dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   }
   return r == CUDA_SUCCESS;
 }
@@ -421,7 +401,7 @@ bool make_map(const BornArgs& a, bool zpass, CUtensorMap* m, bool b16 = false) {
 template <int R2, int KIND>
 cudaError_t launch_kind(const BornArgs& a, int jj, const DevFft& f, int* fault, cudaStream_t s) {
   using L = ColSmem<kR1 * R2>;
-  constexpr size_t smem = KIND == 3 ? L::kTotalZ16 : KIND == 2 ? L::kTotalZ : L::kTotalY;
+  constexpr size_t smem = KIND == 3 ? L::kTotalZ16 : L::kTotalY;
   static DeviceFlags configured;   // attribute raised once per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -433,12 +413,12 @@ cudaError_t launch_kind(const BornArgs& a, int jj, const DevFft& f, int* fault, 
     configured.set(dev);
   }
   CUtensorMap map;
-  if (!make_map(a, KIND >= 2, &map, KIND == 3)) return cudaErrorInvalidValue;
+  if (!make_map(a, &map, KIND == 3)) return cudaErrorInvalidValue;
   int nsm = 0;
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const int nxt = (a.px + kW - 1) / kW;
-  const long long nout = KIND >= 2 ? (long long)a.py * a.nbatch : (long long)a.pz * a.nbatch;
+  const long long nout = KIND == 3 ? (long long)a.py * a.nbatch : (long long)a.pz * a.nbatch;
   const long long ntiles = nout * nxt;
   int per_sm = 0;   // resident CTAs per SM (shared memory and registers allowing)
   constexpr int nthr = threads_of<KIND>();
@@ -456,11 +436,11 @@ cudaError_t dispatch(const BornArgs& a, int jj, const DevFft& f, int* fault, cud
   switch (f.plan.n / kR1) {
     case 11: return launch_kind<11, KIND>(a, jj, f, fault, s);
     case 12:   // z-pass only (96 = 8 x 12, the fused passes' even length)
-      if constexpr (KIND >= 2) return launch_kind<12, KIND>(a, jj, f, fault, s);
+      if constexpr (KIND == 3) return launch_kind<12, KIND>(a, jj, f, fault, s);
       return cudaErrorNotSupported;
     case 13: case 14: case 16: case 17: case 18: case 20:
       // z-pass only (104 - 160-point columns behind the fused xy-pass)
-      if constexpr (KIND >= 2) {
+      if constexpr (KIND == 3) {
         switch (f.plan.n / kR1) {
           case 13: return launch_kind<13, KIND>(a, jj, f, fault, s);
           case 14: return launch_kind<14, KIND>(a, jj, f, fault, s);
@@ -502,11 +482,8 @@ cudaError_t launch_fft_y_pipe(const BornArgs& a, bool inverse, const DevFft& fy,
 }
 
 cudaError_t launch_born_z_pipe(const BornArgs& a, int jj, const DevFft& fz, int* fault, cudaStream_t s) {
-  if (a.storage) {
-    if (a.px % 8 != 0) return cudaErrorInvalidValue;   // 8-column exponent blocks, 16-byte rows
-    return dispatch<3>(a, jj, fz, fault, s);
-  }
-  return dispatch<2>(a, jj, fz, fault, s);
+  if (!a.storage || a.px % 8 != 0) return cudaErrorInvalidValue;   // 8-column exponent blocks, 16-byte rows
+  return dispatch<3>(a, jj, fz, fault, s);
 }
 
 }  // namespace odt

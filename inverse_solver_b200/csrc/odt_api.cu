@@ -616,7 +616,12 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   const bool any = H.any_loop();
   const bool pipe_x = !any && !ten && H.use_pipe && born_x_pipe_supported(a, H.fx);
   const bool pipe_y = !any && H.use_pipe && cols_pipe_supported(a, H.fy, false);
-  const bool pipe_z = !any && !vec && H.use_pipe && cols_pipe_supported(a, H.fz, true);
+  // 16-bit storage keeps its own z-pass (set up below); the others share one
+  const bool b16 = H.storage == ODT_STORAGE_B16;
+  const bool pipe_z = !any && !vec && H.use_pipe &&
+                      (b16 ? cols_pipe_supported(a, H.fz, true) : z_pass_supported(a, H.fz));
+  // (reported as born_z_pipe on 8 R points, R of the 16-bit pass; as born_z elsewhere)
+  const int zkind = pipe_z && cols_pipe_supported(a, H.fz, true) ? kKBornZPipe : kKBornZ;
   DyadArgs dy{};
   if (vec) {
     for (int i = 0; i < 3; ++i) dy.rad[i] = P.rad[i];
@@ -627,7 +632,7 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   // or generic, reads its permuted x-y spectrum): scalar potentials
   const bool fused_xy = !any && !ten && !vec && H.use_pipe && H.use_xy && B >= 1 && born_xy_supported(a, H.max_smem);
   a.perm_xy = fused_xy ? 1 : 0;
-  if (H.storage == ODT_STORAGE_B16) {
+  if (b16) {
     if (!fused_xy || !pipe_z)
       raise(ODT_ERR_UNSUPPORTED,
             "16-bit block storage (ODT_STORAGE_B16) needs the fused xy-pass: a scalar potential on a grid "
@@ -651,9 +656,11 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     H.mark_begin(jj == j0 || (a.storage && jj <= 4) ? kKBornXYEdge : kKBornXY, s);
     ODT_CUDA(launch_born_xy(a, jj == j0 ? kBornFirst : kBornMid, jj, H.fx, s));
     H.mark_end(s);
-    H.mark_begin(pipe_z ? kKBornZPipe : kKBornZ, s);
-    if (pipe_z)
+    H.mark_begin(zkind, s);
+    if (pipe_z && b16)
       ODT_CUDA(launch_born_z_pipe(a, jj, H.fz, H.d_fault, s));
+    else if (pipe_z)
+      ODT_CUDA(launch_z_pass(a, jj, H.fz, H.d_fault, s));
     else
       ODT_CUDA(launch_born_z(a, jj, H.fz, s));
     H.mark_end(s);
@@ -683,11 +690,11 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     else
       ODT_CUDA(launch_fft_cols(a.T, a.T, a.px, (long long)a.pz * nbp, 0, 0, 1.0f, false, H.fy, s));
     H.mark_end(s);
-    H.mark_begin(pipe_z ? kKBornZPipe : kKBornZ, s);
+    H.mark_begin(zkind, s);
     if (vec)
       ODT_CUDA(launch_born_z_dyadic(a, dy, jj, H.fz, H.max_smem, s));
     else if (pipe_z)
-      ODT_CUDA(launch_born_z_pipe(a, jj, H.fz, H.d_fault, s));
+      ODT_CUDA(launch_z_pass(a, jj, H.fz, H.d_fault, s));
     else
       ODT_CUDA(launch_born_z(a, jj, H.fz, s));
     H.mark_end(s);
