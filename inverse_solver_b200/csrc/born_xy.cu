@@ -1,7 +1,8 @@
 // Fused xy-pass of the Born iteration: the whole x-y plane of one z and one
-// illumination in shared memory, so one iteration moves 72 bytes per voxel
-// (this pass: T, Field_n, Field read and written, V read; the z-pass: T read
-// and written) instead of the 104 of separate x-, y- and y-passes.
+// illumination in shared memory, so one iteration moves 61 bytes per voxel
+// (this pass: T and X read and written, the incident field read inside the
+// ROI, V read; the z-pass: T read and written) instead of the 93 of separate
+// x-, y- and y-passes.
 //
 // Per plane (FORWARD_SOLVER_CONVERGENT_BORN.m:577-647; jj = iteration):
 //   inverse y-FFT and inverse x-FFT of the spectral array T (the last two
@@ -11,7 +12,7 @@
 // The z-pass (cols_pipe.cu) does the z-FFT, the Green's multiply and the
 // inverse z-FFT in between.
 //
-// Transforms along an axis of length N = 8 R (11 <= R <= 20): index
+// Transforms along an axis of length N = 8 R (5 <= R <= 28): index
 // n = R n1 + n2 (n1 < 8, n2 < R), k = k1 + 8 k2 (k1 < 8, k2 < R).
 //   forward  F1: 8-point DFT over n1 of the positions R n1 + n2 (stride R),
 //                result k1 stored at R k1 + n2;
@@ -24,22 +25,22 @@
 // (spectral index k1 + 8 k2 at position R k1 + k2 along x and along y) and
 // the z-pass maps each column to its (kx, ky) accordingly (BornArgs.perm_xy).
 // Space-domain data is in natural order, so the pointwise work reads and
-// writes Field_n / Field / V / the incident field in their global layout.
+// writes X / V / the incident field in their global layout.
 //
 // Seven steps per plane:
 //   1 y-F3^-1 + F2^-1  read T from global (one R-point column group per item)
 //   2 y-F1^-1          shared memory
 //   3 x-F3^-1 + F2^-1  shared memory
 //   4 x-F1^-1, update + source, x-F1 (8 points per item; the global reads
-//                      and writes of Field_n, Field, V, E_inc)
+//                      and writes of X, V, E_inc)
 //   5 x-F2 + F3        shared memory
 //   6 y-F1             shared memory
 //   7 y-F2 + F3        write T to global
-// One CTA per SM (the plane takes 8 N^2 bytes: 185 KB for N = 152) with 32 R
-// threads -- R warps -- persistent over the planes (illumination fastest, so
-// concurrent CTAs share V's planes in L2; prefetching the next plane's T,
-// Field_n and Field into L2 with cp.async.bulk.prefetch made a step 5.4 ms
-// slower, so there is none).  Steps 2-6 touch, for one n2, only
+// One CTA (or a pair, see xy_ctas) per plane (8 N^2 bytes: 185 KB for N = 152)
+// with 32 R threads -- R warps -- persistent over the planes (illumination fastest, so
+// concurrent CTAs share V's planes in L2; prefetching the next plane's arrays
+// into L2 with cp.async.bulk.prefetch made a step 5.4 ms slower, so there is
+// none).  Steps 2-6 touch, for one n2, only
 // the 8 rows R n1 + n2 (step 2 and 6 combine exactly those rows, steps 3-5
 // work along rows), so warp w takes n2 = w and runs steps 2-6 on its own rows
 // with warp-level synchronisation only; step 7 of a plane and step 1 of the
@@ -71,8 +72,26 @@ namespace {
 constexpr size_t a16(size_t b) { return (b + 15) & ~(size_t)15; }
 constexpr size_t a128(size_t b) { return (b + 127) & ~(size_t)127; }
 
+// CTAs per plane.  Planes of 168 to 224 points (226 to 416 KB) take a cluster
+// of two, CTA c with the rows R n1 + n2 of its half of the n2.  Steps 2-6 work
+// on the rows of one n2, so only steps 1 and 7 (one R-point column group per
+// item) cross to the other CTA, through distributed shared memory, and the two
+// barriers per plane become cluster barriers.  216 points, 192 x 192 x 96, 8
+// illuminations: 0.69 ms per launch against 0.80 ms of the separate x-pass and
+// two y-passes it replaces; clusters of four with two CTAs per SM measured
+// 0.72 ms.
+// Planes of 112 to 160 points with an even R take the pair as well, two CTAs
+// per SM, so that one plane's transforms overlap another's loads: 0.526 ->
+// 0.499 ms at 160 points, 0.373 -> 0.354 at 144, 0.250 -> 0.240 at 128 (16
+// illuminations).  An odd R splits unevenly (19 of 20 warps) and lost: 0.397
+// -> 0.479 ms at 152 points, 0.239 -> 0.248 at 120.
+constexpr int kMaxR16 = 20;   // largest R of the 16-bit storage
+constexpr int xy_ctas(int r) { return r > 20 || (r >= 14 && r % 2 == 0) ? 2 : 1; }
+
 template <int R>
 struct XYSmem {
+  static constexpr int C = xy_ctas(R);
+  static constexpr int H = (R + C - 1) / C;   // values of n2 (warps) per CTA
   static constexpr int N = 8 * R;
   static constexpr size_t kTw = 0;                                    // W_N^k, k < N
   static constexpr size_t kRampX = kTw + a16(sizeof(float2) * N);     // ramp along x
@@ -90,7 +109,7 @@ struct XYSmem {
   // different banks ((R + 1) k1) and the pitch N + N / R is 8 mod 16 again
   static constexpr bool kPad = R % 2 == 0;
   static constexpr int P = kPad ? N + N / R : N;
-  static constexpr size_t kTotal = kPlane + sizeof(float2) * N * P;
+  static constexpr size_t kTotal = kPlane + sizeof(float2) * 8 * H * P;
   // in-row position of x
   static __device__ __forceinline__ int sx(int x) { return kPad ? x + x / R : x; }
 };
@@ -100,6 +119,23 @@ struct XYSmem {
 // the 16-bit storage's term-by-term series only (its iterations 2-4)
 enum XYKind { kXYSteady = 0, kXYEarly = 1, kXYFinal = 2, kXYFirst = 3 };
 
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// p of CTA `rank` of the cluster, as a generic address
+__device__ __forceinline__ float2* cluster_ptr(float2* p, unsigned rank) {
+  unsigned long long q;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"((unsigned long long)p), "r"(rank));
+  return reinterpret_cast<float2*>(q);
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+#endif
+
 // (i c) * v for real c: (-c v.y, c v.x), two products (a complex product
 // with (0, c) would also form 0 * v.x and 0 * v.y)
 __device__ __forceinline__ float2 mul_i(float c, float2 v) { return make_float2(-(c * v.y), c * v.x); }
@@ -107,18 +143,28 @@ __device__ __forceinline__ float2 mul_i(float c, float2 v) { return make_float2(
 // ST: storage of T and Field_n, 0 = complex64, 1 = 16-bit block floating
 // point (b16.cuh; T's blocks are 8 consecutive x of a row, Field_n's are the
 // values of one n1 in 8 consecutive step-4 work items of a warp, exponent
-// index plane * N^2/8 + n1 * R^2 + w * R + item / 8)
+// index plane * N^2/8 + n1 * R^2 + n2 * R + item / 8)
 // __launch_bounds__ lets the compiler fit the R warps of the one CTA per SM
 // into the register file, which is split into four quarters of 16384
 // registers (one per warp scheduler): 19 warps put five warps on a quarter,
 // so at most 96 registers per thread for R = 19 (104 did not launch).
+// Small planes: several CTAs per SM as far as registers for step 4 (about 80)
+// and shared memory allow, so that one CTA's transforms overlap another's
+// loads (88 points, 16 illuminations: 62 Gvoxel-iterations/s of the loop; 56
+// to 80 points ran on the separate generic tiles before).
+template <int R>
+constexpr int xy_min_ctas() {
+  return R <= 6 ? 4 : R <= 8 ? 3 : R <= 12 || (xy_ctas(R) == 2 && R <= 20) ? 2 : 1;
+}
+
 template <int R, int KIND, int ST>
-__global__ void __launch_bounds__(32 * R, 1)
+__global__ void __launch_bounds__(32 * XYSmem<R>::H, xy_min_ctas<R>())
     born_xy_kernel(const BornArgs a, const int jj, const float2* __restrict__ twg, const int nplanes) {
 #if defined(__CUDA_ARCH__)
   constexpr int N = 8 * R;
-  constexpr int NT = 32 * R;
   using L = XYSmem<R>;
+  constexpr int C = L::C, H = L::H;
+  constexpr int NT = 32 * H;
   extern __shared__ __align__(128) unsigned char sm[];
   float2* tw = reinterpret_cast<float2*>(sm + L::kTw);
   float2* rxt = reinterpret_cast<float2*>(sm + L::kRampX);
@@ -128,7 +174,29 @@ __global__ void __launch_bounds__(32 * R, 1)
   float2* twk = reinterpret_cast<float2*>(sm + L::kTk);
   float2* pl = reinterpret_cast<float2*>(sm + L::kPlane);
   const int tid = threadIdx.x;
-  const int w = tid >> 5, lane = tid & 31;   // warp w owns the rows R n1 + w in steps 2-6
+  // warp w owns the rows R n1 + n2, n2 = wn, in steps 2-6; they are the rows
+  // H n1 + w of this CTA's buffer
+  const int w = tid >> 5, lane = tid & 31;
+  const int rank = C == 1 ? 0 : (int)cluster_rank();
+  const int wn = H * rank + w;
+  const bool mine = C == 1 || wn < R;   // an odd R leaves the second CTA's last warp without rows
+  float2* peer[C];
+  if constexpr (C == 1) {
+    peer[0] = pl;
+  } else {
+#pragma unroll
+    for (int q = 0; q < C; ++q) peer[q] = cluster_ptr(pl, q);
+  }
+  // element (row R k1 + r, x) of the plane, r known at compile time
+  auto at = [&](int k1, int r, int sxx) -> float2& {
+    if constexpr (C == 1) return pl[(R * k1 + r) * L::P + sxx];
+    else return peer[r / H][(H * k1 + r % H) * L::P + sxx];
+  };
+  auto plane_sync = [] {
+    if constexpr (C == 1) __syncthreads();
+    else cluster_barrier();
+  };
+  const int item0 = tid + rank * NT;   // items of steps 1 and 7 over both CTAs
   const float2 one = make_float2(1.f, 0.f);
   const float2 z2 = make_float2(0.f, 0.f);
   for (int i = tid; i < N; i += NT) {
@@ -182,19 +250,21 @@ __global__ void __launch_bounds__(32 * R, 1)
 #pragma unroll
     for (int r = 1; r < R; ++r) v[r] = cmul(v[r], cconj(tw[r * k1]));
 #pragma unroll
-    for (int r = 0; r < R; ++r) pl[(R * k1 + r) * L::P + L::sx(x)] = v[r];
+    for (int r = 0; r < R; ++r) at(k1, r, L::sx(x)) = v[r];
   };
   // Step 7 of item (x, k1) reads the rows R k1 + r of column x and step 1 of
   // the same item writes them, with the same item -> thread map: a thread
   // goes from its step-7 item of one plane straight to its step-1 item of
   // the next, with no CTA barrier in between.
   bool loaded = false;   // step 1 of this plane done during the previous plane's step 7
-  for (int p = blockIdx.x; p < nplanes; p += gridDim.x) {
+  const int pstride = gridDim.x / C;
+  if constexpr (C > 1) cluster_barrier();   // the other CTA has started before its buffer is written
+  for (int p = blockIdx.x / C; p < nplanes; p += pstride) {
     const int b = p % a.nbatch;
     const int z = p / a.nbatch;
     const long long g0 = plane_n * (z + (long long)a.pz * b);   // plane (z, b) of T / Field_n / Field
     const long long v0 = plane_n * z;
-    const int pn = p + gridDim.x;
+    const int pn = p + pstride;
     const long long gn = pn < nplanes ? plane_n * (pn / a.nbatch + (long long)a.pz * (pn % a.nbatch)) : -1;
     const float mz = a.mask[2][z];
     const float2 rz = a.acyclic ? a.ramp[2][z] : one;
@@ -203,22 +273,22 @@ __global__ void __launch_bounds__(32 * R, 1)
     if constexpr (kInv) {
       // ---- 1 (unless the previous plane's step 7 did it item by item)
       if (!loaded)
-        for (int i = tid; i < 8 * N; i += NT) step1(i, g0);
-      __syncthreads();
+        for (int i = item0; i < 8 * N; i += C * NT) step1(i, g0);
+      plane_sync();
       // ---- 2: y-F1^-1 (8-point over k1 at rows R k1 + w) -> natural rows R n1 + w
-      for (int x = lane; x < N; x += 32) {
+      for (int x = lane; mine && x < N; x += 32) {
         float2 v[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = pl[(R * r + w) * L::P + L::sx(x)];
+        for (int r = 0; r < 8; ++r) v[r] = pl[(H * r + w) * L::P + L::sx(x)];
         Butterfly<8, true>::run(v, tw, N);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) pl[(R * r + w) * L::P + L::sx(x)] = v[r];
+        for (int r = 0; r < 8; ++r) pl[(H * r + w) * L::P + L::sx(x)] = v[r];
       }
       __syncwarp();
       // ---- 3: x-F3^-1 + F2^-1 on the contiguous groups R k1 .. R k1 + R-1 of the warp's rows
-      for (int it = lane; it < 64; it += 32) {
-        const int k1 = it & 7, y = R * (it >> 3) + w;
-        float2* row = pl + y * L::P + (R + (L::kPad ? 1 : 0)) * k1;
+      for (int it = lane; mine && it < 64; it += 32) {
+        const int k1 = it & 7;
+        float2* row = pl + (H * (it >> 3) + w) * L::P + (R + (L::kPad ? 1 : 0)) * k1;
         float2 v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = row[r];
@@ -234,12 +304,12 @@ __global__ void __launch_bounds__(32 * R, 1)
 
     // ---- 4: x-F1^-1 -> update of iteration jj-1 and source of jj -> x-F1, on
     //      the warp's rows (item it: row R (it / R) + w, n2 = it % R)
-    for (int it = lane; it < 8 * R; it += 32) {
-      const int n2 = it % R, y = R * (it / R) + w;
+    for (int it = lane; mine && it < 8 * R; it += 32) {
+      const int n2 = it % R, y = R * (it / R) + wn;
       // Field_n's exponent block of this item's n1 = r value: the 8 lanes of a
       // group (8 consecutive it) share one; block w R + it / 8 of n1's R^2
-      const long long fe = (g0 >> 3) + w * R + (it >> 3);
-      float2* row = pl + y * L::P;
+      const long long fe = (g0 >> 3) + wn * R + (it >> 3);
+      float2* row = pl + (H * (it / R) + w) * L::P;
       const long long gy = g0 + (long long)y * N;
       const long long vy = v0 + (long long)y * N;
       const bool yzroi = zroi && (unsigned)(y - a.ry0) < (unsigned)a.ry;
@@ -355,15 +425,15 @@ __global__ void __launch_bounds__(32 * R, 1)
       }
     }
     if constexpr (!kFwd) {
-      __syncthreads();   // the next plane's step 1 overwrites the plane
+      plane_sync();   // the next plane's step 1 overwrites the plane
       loaded = false;
       continue;
     }
     __syncwarp();
     // ---- 5: x-F2 + F3 on the contiguous groups of the warp's rows
-    for (int it = lane; it < 64; it += 32) {
-      const int k1 = it & 7, y = R * (it >> 3) + w;
-      float2* row = pl + y * L::P + (R + (L::kPad ? 1 : 0)) * k1;
+    for (int it = lane; mine && it < 64; it += 32) {
+      const int k1 = it & 7;
+      float2* row = pl + (H * (it >> 3) + w) * L::P + (R + (L::kPad ? 1 : 0)) * k1;
       float2 v[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = row[r];
@@ -376,21 +446,21 @@ __global__ void __launch_bounds__(32 * R, 1)
     }
     __syncwarp();
     // ---- 6: y-F1 (8-point over n1 at the warp's rows R n1 + w)
-    for (int x = lane; x < N; x += 32) {
+    for (int x = lane; mine && x < N; x += 32) {
       float2 v[8];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) v[r] = pl[(R * r + w) * L::P + L::sx(x)];
+      for (int r = 0; r < 8; ++r) v[r] = pl[(H * r + w) * L::P + L::sx(x)];
       Butterfly<8, false>::run(v, tw, N);
 #pragma unroll
-      for (int r = 0; r < 8; ++r) pl[(R * r + w) * L::P + L::sx(x)] = v[r];
+      for (int r = 0; r < 8; ++r) pl[(H * r + w) * L::P + L::sx(x)] = v[r];
     }
-    __syncthreads();
+    plane_sync();
     // ---- 7: y-F2 + F3 -> T
-    for (int i = tid; i < 8 * N; i += NT) {
+    for (int i = item0; i < 8 * N; i += C * NT) {
       const int x = i % N, k1 = i / N;
       float2 v[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = pl[(R * k1 + r) * L::P + L::sx(x)];
+      for (int r = 0; r < R; ++r) v[r] = at(k1, r, L::sx(x));
 #pragma unroll
       for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[r * k1]);
       Butterfly<R, false>::run(v, tw, N);
@@ -412,9 +482,11 @@ __global__ void __launch_bounds__(32 * R, 1)
       }
     }
     if (kInv && gn >= 0)   // the same items as this thread's step 7: no barrier needed
-      for (int i = tid; i < 8 * N; i += NT) step1(i, gn);
+      for (int i = item0; i < 8 * N; i += C * NT) step1(i, gn);
     loaded = kInv && gn >= 0;
-    if (!loaded) __syncthreads();   // the next plane's step 4 (first kind) writes other threads' rows
+    // the next plane's step 4 (first kind) writes other threads' rows, and
+    // after the last plane the other CTA may still read this one's
+    if (!loaded) plane_sync();
   }
 #endif
 }
@@ -435,14 +507,36 @@ cudaError_t launch_r(const BornArgs& a, int jj, const float2* tw, cudaStream_t s
   int nsm = 0;
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;   // the kernel needs one resident CTA per SM
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, born_xy_kernel<R, KIND, ST>, 32 * R, L::kTotal);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   const long long nplanes = (long long)a.pz * a.nbatch;
-  const int grid = (int)(nplanes < nsm ? nplanes : nsm);
-  born_xy_kernel<R, KIND, ST><<<grid, 32 * R, L::kTotal, s>>>(a, jj, tw, (int)nplanes);
-  return cudaGetLastError();
+  if constexpr (L::C == 1) {
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, born_xy_kernel<R, KIND, ST>, 32 * L::H, L::kTotal);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+    const long long cap = (long long)per_sm * nsm;
+    const int grid = (int)(nplanes < cap ? nplanes : cap);
+    born_xy_kernel<R, KIND, ST><<<grid, 32 * L::H, L::kTotal, s>>>(a, jj, tw, (int)nplanes);
+    return cudaGetLastError();
+  } else {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = L::C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(32 * L::H);
+    cfg.gridDim = dim3((unsigned)(nsm * xy_min_ctas<R>()) / L::C * L::C);
+    cfg.dynamicSmemBytes = L::kTotal;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;   // resident at once (SMs that find no partner stay idle)
+    e = cudaOccupancyMaxActiveClusters(&clusters, born_xy_kernel<R, KIND, ST>, &cfg);
+    if (e != cudaSuccess) return e;
+    if (clusters < 1) return cudaErrorLaunchOutOfResources;
+    cfg.gridDim = dim3((unsigned)(nplanes < clusters ? nplanes : clusters) * L::C);
+    return cudaLaunchKernelEx(&cfg, born_xy_kernel<R, KIND, ST>, a, jj, tw, (int)nplanes);
+  }
 }
 
 template <int R, int ST>
@@ -459,32 +553,32 @@ cudaError_t launch_kind_st(const BornArgs& a, int kind, int jj, const float2* tw
 
 template <int R>
 cudaError_t launch_kind(const BornArgs& a, int kind, int jj, const float2* tw, cudaStream_t s) {
-  return a.storage ? launch_kind_st<R, 1>(a, kind, jj, tw, s) : launch_kind_st<R, 0>(a, kind, jj, tw, s);
+  if constexpr (R >= 11 && R <= kMaxR16)
+    if (a.storage) return launch_kind_st<R, 1>(a, kind, jj, tw, s);
+  return a.storage ? cudaErrorNotSupported : launch_kind_st<R, 0>(a, kind, jj, tw, s);
 }
 
 }  // namespace
 
-bool born_xy_supported(const BornArgs& a, int max_smem) {
+// radices of the fused pass (16-bit storage: 11 to 20)
+#define ODT_XY_LIST(X)                                                                                     \
+  X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19) X(20) X(21) X(22) X(23) \
+  X(24) X(25) X(26) X(27) X(28)
+
+bool born_xy_supported(const BornArgs& a, int max_smem, bool b16) {
   if (a.px != a.py || a.px % 8 != 0) return false;
   const int r = a.px / 8;
+  if (b16 && (r < 11 || r > kMaxR16)) return false;
   size_t need = 0;
   switch (r) {
-    case 11: need = XYSmem<11>::kTotal; break;
-    case 12: need = XYSmem<12>::kTotal; break;
-    case 13: need = XYSmem<13>::kTotal; break;
-    case 14: need = XYSmem<14>::kTotal; break;
-    case 15: need = XYSmem<15>::kTotal; break;
-    case 16: need = XYSmem<16>::kTotal; break;
-    case 17: need = XYSmem<17>::kTotal; break;
-    case 18: need = XYSmem<18>::kTotal; break;
-    case 19: need = XYSmem<19>::kTotal; break;
-    case 20: need = XYSmem<20>::kTotal; break;
+#define ODT_XY_CASE(R) \
+  case R: need = XYSmem<R>::kTotal; break;
+    ODT_XY_LIST(ODT_XY_CASE)
+#undef ODT_XY_CASE
     default: return false;
   }
   return need <= (size_t)max_smem && (long long)a.pz * a.nbatch < (1LL << 31);
 }
-
-int born_xy_perm_radix(const BornArgs& a) { return a.px / 8; }
 
 cudaError_t launch_born_xy(const BornArgs& a, int mode, int jj, const DevFft& fx, cudaStream_t s) {
   int kind;
@@ -493,16 +587,10 @@ cudaError_t launch_born_xy(const BornArgs& a, int mode, int jj, const DevFft& fx
   else kind = a.storage && jj <= 4 ? kXYEarly : kXYSteady;   // 16-bit steady: e >= 4 (Field += Field_n only)
   if (mode == kBornFirst ? jj > (a.storage ? 1 : 2) : jj < 2) return cudaErrorInvalidValue;
   switch (a.px / 8) {
-    case 11: return launch_kind<11>(a, kind, jj, fx.tw, s);
-    case 12: return launch_kind<12>(a, kind, jj, fx.tw, s);
-    case 13: return launch_kind<13>(a, kind, jj, fx.tw, s);
-    case 14: return launch_kind<14>(a, kind, jj, fx.tw, s);
-    case 15: return launch_kind<15>(a, kind, jj, fx.tw, s);
-    case 16: return launch_kind<16>(a, kind, jj, fx.tw, s);
-    case 17: return launch_kind<17>(a, kind, jj, fx.tw, s);
-    case 18: return launch_kind<18>(a, kind, jj, fx.tw, s);
-    case 19: return launch_kind<19>(a, kind, jj, fx.tw, s);
-    case 20: return launch_kind<20>(a, kind, jj, fx.tw, s);
+#define ODT_XY_CASE(R) \
+  case R: return launch_kind<R>(a, kind, jj, fx.tw, s);
+    ODT_XY_LIST(ODT_XY_CASE)
+#undef ODT_XY_CASE
     default: return cudaErrorNotSupported;
   }
 }

@@ -135,7 +135,7 @@ cudaError_t launch_z_pass(const BornArgs& a, int jj, const DevFft& fz, int* faul
 // 15, 19}; replaces launch_born_x and both y-FFTs (modes as launch_born_x;
 // the z-pass must run with a.perm_xy = 1).  Same results as the separate passes
 // up to the order of the FFT arithmetic.
-bool born_xy_supported(const BornArgs& a, int max_smem);
+bool born_xy_supported(const BornArgs& a, int max_smem, bool b16);
 cudaError_t launch_born_xy(const BornArgs& a, int mode, int jj, const DevFft& fx, cudaStream_t s);
 // z-pass of iteration jj: forward z-FFT, Green's multiply, inverse z-FFT.
 cudaError_t launch_born_z(const BornArgs& a, int jj, const DevFft& fz, cudaStream_t s);

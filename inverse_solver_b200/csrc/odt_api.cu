@@ -628,9 +628,9 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     dy.absorb = make_float2(P.pp.absorb.re, P.pp.absorb.im);
   }
   const long long xlines = (long long)a.py * a.pz * nbp;
-  // fused xy-pass (x- and both y-passes in one kernel; the z-pass, pipelined
-  // or generic, reads its permuted x-y spectrum): scalar potentials
-  const bool fused_xy = !any && !ten && !vec && H.use_pipe && H.use_xy && B >= 1 && born_xy_supported(a, H.max_smem);
+  // fused xy-pass (x- and both y-passes in one kernel; the z-pass, pipelined,
+  // dyadic or generic, reads its permuted x-y spectrum): scalar potentials
+  const bool fused_xy = !any && !ten && H.use_pipe && H.use_xy && B >= 1 && born_xy_supported(a, H.max_smem, b16);
   a.perm_xy = fused_xy ? 1 : 0;
   if (b16) {
     if (!fused_xy || !pipe_z)
@@ -657,7 +657,9 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     ODT_CUDA(launch_born_xy(a, jj == j0 ? kBornFirst : kBornMid, jj, H.fx, s));
     H.mark_end(s);
     H.mark_begin(zkind, s);
-    if (pipe_z && b16)
+    if (vec)
+      ODT_CUDA(launch_born_z_dyadic(a, dy, jj, H.fz, H.max_smem, s));
+    else if (pipe_z && b16)
       ODT_CUDA(launch_born_z_pipe(a, jj, H.fz, H.d_fault, s));
     else if (pipe_z)
       ODT_CUDA(launch_z_pass(a, jj, H.fz, H.d_fault, s));
@@ -1521,7 +1523,8 @@ odt_status odt_autotune(odt_handle h, int32_t n_ill, odt_tune_result* out) {
     probe.py = H->g.sim_size[1];
     probe.pz = H->g.sim_size[2];
     probe.nbatch = nb * H->np;
-    const bool xy_ok = H->np == 1 && !H->pot[0].tensor && born_xy_supported(probe, H->max_smem);
+    const bool xy_ok = !H->pot[0].tensor && !H->any_loop() &&
+                       born_xy_supported(probe, H->max_smem, H->storage == ODT_STORAGE_B16);
     const bool saved_xy = H->use_xy, saved_pipe = H->use_pipe;
     const bool want_t = H->ktrans != nullptr;
     cudaEvent_t e0, e1;
