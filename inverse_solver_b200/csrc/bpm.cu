@@ -26,6 +26,7 @@
 #include "../../include/odt.h"
 #include "cbs_kernels.cuh"
 #include "scratch.cuh"
+#include "tile_bodies.cuh"
 
 namespace odt {
 const char* set_last_error(const std::string& msg);  // odt_api.cu
@@ -327,6 +328,216 @@ bpm_march128_kernel(float2* __restrict__ fld, const float2* __restrict__ rk, con
   }
 }
 
+// ---- two fused passes per slice, any plane the tile transforms cover
+// Between slices the planes are kept transformed along x only:
+//   cols : forward y-FFT, * refocus_kernel, inverse y-FFT
+//   lines: inverse x-FFT, * (1/N) exp(field_multiplier(:,:,z) * inv_cos),
+//          forward x-FFT (not after the last slice, whose fft2 / ifft2 pair
+//          cancels)
+// so a slice is two launches and 32 bytes per element, where separate
+// products and transforms took six launches and 96 bytes.  The planes of a
+// call (a few MB) stay in L2: the passes are bound by launch and barrier
+// latency, so tiles are 4 to 16 pencils, the largest that still give every
+// SM three CTAs.
+constexpr int kTileThreads = 128;
+
+struct PhaseOp {   // on the values x = j + r nb of line c
+  const float2* fz;   // field multiplier of the slice [n1, n2]
+  const float* inv_cos;
+  long long line0;
+  int n1, n2;
+  float inv_n;
+  long long nlines;
+  template <int R>
+  __device__ __forceinline__ void apply(int c, int j, int nb, float2* v) const {
+    const long long L = lmin(line0 + c, nlines - 1);
+    const int y = (int)(L % n2);
+    const float ic = inv_cos ? inv_cos[L / n2] : 1.f;
+    float2 e[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) e[r] = fz[(long long)y * n1 + j + r * nb];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (inv_cos) e[r] = cscale(e[r], ic);
+      float sn, cs;
+      sincosf(e[r].y, &sn, &cs);
+      const float m = expf(e[r].x);
+      v[r] = cmul(cscale(v[r], inv_n), make_float2(m * cs, m * sn));
+    }
+  }
+};
+
+struct RefocusOp {   // on the values ky = j + r nb of column c
+  const float2* rk;   // refocus kernel at column 0 of the tile, row pitch n1
+  int n1, ncol;
+  template <int R>
+  __device__ __forceinline__ void apply(int c, int j, int nb, float2* v) const {
+    if (c >= ncol) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = cmul(v[r], rk[(long long)(j + r * nb) * n1 + c]);
+  }
+};
+
+// stores a last pass's values (after the op) in natural order
+template <class G, class Op>
+struct StoreOp {
+  Op op;
+  G g;
+  template <int R>
+  __device__ __forceinline__ void apply(int c, int j, int nb, float2* v) const {
+    op.template apply<R>(c, j, nb, v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) g.store(j + r * nb, c, v[r]);
+  }
+};
+
+template <int CLS>
+__global__ void __launch_bounds__(kTileThreads)
+bpm_lines_kernel(float2* __restrict__ fld, PhaseOp op, const FftPlan plan, const float2* __restrict__ twg, const int W,
+                 const int last) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const Thr th{(int)threadIdx.x, (int)blockDim.x};
+  const int n = plan.n, ld = smem_line_ld(n), P = plan.npass;
+  float2* tw = reinterpret_cast<float2*>(smraw);
+  SmemLine cur{reinterpret_cast<float2*>(smraw + align16(sizeof(float2) * n)), ld};
+  SmemLine oth{cur.s + (size_t)W * ld, ld};
+  load_twiddles(th, tw, twg, n);
+  op.line0 = (long long)blockIdx.x * W;
+  const int nl = (int)lmin(W, op.nlines - op.line0);
+  float2* base = fld + op.line0 * n;
+  const GlobalPlain g{base, base, 1, n, nl};
+  const LineMap m{W};
+  __syncthreads();
+  int ns = 1;   // inverse passes, radices f[P-1] .. f[1]
+  for (int i = 0; i + 1 < P; ++i) {
+    const int R = plan.radix[P - 1 - i];
+    if (i == 0) tile_pass_any<CLS, true>(th, R, m, n, ns, tw, g, cur);
+    else tile_pass_any<CLS, true>(th, R, m, n, ns, tw, oth, cur);
+    __syncthreads();
+    ns *= R;
+    const SmemLine t = cur;
+    cur = oth;
+    oth = t;
+  }
+  const int R0 = plan.radix[0];
+  if (last) {
+    const StoreOp<GlobalPlain, PhaseOp> sop{op, g};
+    if (P == 1) tile_mid_any<CLS, true, kMidEnd>(th, R0, m, n, tw, g, g, sop);
+    else tile_mid_any<CLS, true, kMidEnd>(th, R0, m, n, tw, oth, g, sop);
+    return;
+  }
+  if (P == 1) {
+    tile_mid_any<CLS, true, kMidBoth>(th, R0, m, n, tw, g, g, op);
+    return;
+  }
+  tile_mid_any<CLS, true, kMidBoth>(th, R0, m, n, tw, oth, cur, op);
+  __syncthreads();
+  ns = R0;
+  for (int p = 1; p < P; ++p) {   // forward passes f[1] .. f[P-1]; the last one stores
+    const SmemLine t = cur;
+    cur = oth;
+    oth = t;
+    const int R = plan.radix[p];
+    if (p == P - 1) tile_pass_any<CLS, false>(th, R, m, n, ns, tw, oth, g);
+    else tile_pass_any<CLS, false>(th, R, m, n, ns, tw, oth, cur);
+    __syncthreads();
+    ns *= R;
+  }
+}
+
+template <int CLS>
+__global__ void __launch_bounds__(kTileThreads)
+bpm_cols_kernel(float2* __restrict__ fld, const float2* __restrict__ rk, const int n1, const FftPlan plan,
+                const float2* __restrict__ twg, const int lgW) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const Thr th{(int)threadIdx.x, (int)blockDim.x};
+  const int n = plan.n, W = 1 << lgW, P = plan.npass;
+  float2* tw = reinterpret_cast<float2*>(smraw);
+  SmemCol cur{reinterpret_cast<float2*>(smraw + align16(sizeof(float2) * n)), W + 1};
+  SmemCol oth{cur.s + (size_t)n * (W + 1), W + 1};
+  load_twiddles(th, tw, twg, n);
+  const int ntile = (n1 + W - 1) >> lgW;
+  const int b = blockIdx.x / ntile;
+  const int i0 = (blockIdx.x - b * ntile) << lgW;
+  const int ncol = min(W, n1 - i0);
+  float2* base = fld + (long long)b * n1 * n + i0;
+  const GlobalPlain g{base, base, n1, 1, ncol};
+  const ColMap m{lgW};
+  const RefocusOp op{rk + i0, n1, ncol};
+  __syncthreads();
+  int ns = 1;
+  for (int p = 0; p + 1 < P; ++p) {   // forward passes f[0] .. f[P-2]
+    const int R = plan.radix[p];
+    if (p == 0) tile_pass_any<CLS, false>(th, R, m, n, ns, tw, g, cur);
+    else tile_pass_any<CLS, false>(th, R, m, n, ns, tw, oth, cur);
+    __syncthreads();
+    ns *= R;
+    const SmemCol t = cur;
+    cur = oth;
+    oth = t;
+  }
+  const int RL = plan.radix[P - 1];
+  if (P == 1) {
+    tile_mid_any<CLS, false, kMidBoth>(th, RL, m, n, tw, g, g, op);
+    return;
+  }
+  tile_mid_any<CLS, false, kMidBoth>(th, RL, m, n, tw, oth, cur, op);
+  __syncthreads();
+  ns = RL;
+  for (int i = P - 2; i >= 0; --i) {   // inverse passes f[P-2] .. f[0]; the last one stores
+    const SmemCol t = cur;
+    cur = oth;
+    oth = t;
+    const int R = plan.radix[i];
+    if (i == 0) tile_pass_any<CLS, true>(th, R, m, n, ns, tw, oth, g);
+    else tile_pass_any<CLS, true>(th, R, m, n, ns, tw, oth, cur);
+    __syncthreads();
+    ns *= R;
+  }
+}
+
+// log2 of the pencils per tile: the most of 16, 8, 4 (transforms above 512
+// points: 8, 4) that give 3 CTAs per SM, else 4
+int tile_lg(int n, long long pencils) {
+  int lg = n <= 512 ? 4 : n <= 1280 ? 3 : 2;
+  while (lg > 2 && (pencils >> lg) < 3 * 148) --lg;
+  return lg;
+}
+
+#define BPM_CLS(f, K, ...)                                              \
+  switch (f.plan.rclass) {                                              \
+    case 0: return K<0>(__VA_ARGS__);                                   \
+    case 1: return K<1>(__VA_ARGS__);                                   \
+    case 2: return K<2>(__VA_ARGS__);                                   \
+    default: return K<3>(__VA_ARGS__);                                  \
+  }
+
+template <int CLS>
+cudaError_t run_lines_c(float2* fld, const PhaseOp& op, const DevFft& f, int last, cudaStream_t s) {
+  const int W = 1 << tile_lg(f.plan.n, op.nlines);
+  const size_t sm = align16(sizeof(float2) * f.plan.n) + 2 * sizeof(float2) * (size_t)W * smem_line_ld(f.plan.n);
+  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(bpm_lines_kernel<CLS>), sm);
+  if (e != cudaSuccess) return e;
+  bpm_lines_kernel<CLS><<<(unsigned)((op.nlines + W - 1) / W), kTileThreads, sm, s>>>(fld, op, f.plan, f.tw, W, last);
+  return cudaGetLastError();
+}
+cudaError_t run_lines(float2* fld, const PhaseOp& op, const DevFft& f, int last, cudaStream_t s) {
+  BPM_CLS(f, run_lines_c, fld, op, f, last, s)
+}
+
+template <int CLS>
+cudaError_t run_cols_c(float2* fld, const float2* rk, int n1, int nill, const DevFft& f, cudaStream_t s) {
+  const int lg = tile_lg(f.plan.n, (long long)n1 * nill), W = 1 << lg;
+  const size_t sm = align16(sizeof(float2) * f.plan.n) + 2 * sizeof(float2) * (size_t)f.plan.n * (W + 1);
+  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(bpm_cols_kernel<CLS>), sm);
+  if (e != cudaSuccess) return e;
+  bpm_cols_kernel<CLS><<<(unsigned)((n1 + W - 1) / W) * nill, kTileThreads, sm, s>>>(fld, rk, n1, f.plan, f.tw, lg);
+  return cudaGetLastError();
+}
+cudaError_t run_cols(float2* fld, const float2* rk, int n1, int nill, const DevFft& f, cudaStream_t s) {
+  BPM_CLS(f, run_cols_c, fld, rk, n1, nill, f, s)
+}
+
 constexpr size_t kMarchSmem = sizeof(float2) * (kMH * kMP + kM);
 
 odt_status bpm_fail(odt_status st, const std::string& m) {
@@ -416,6 +627,8 @@ extern "C" odt_status odt_bpm_solve(const odt_bpm_args* a) {
   std::string why;
   if (!scratch_fft(B, n1, &f1, &why) || !scratch_fft(B, n2, &f2, &why))
     return bpm_fail(ODT_ERR_UNSUPPORTED, "odt_bpm_solve: " + why);
+  DevFft fl = f1;   // line passes: the small radix at the product (few loads per thread)
+  make_plan(n1, &fl.plan, &why, kSmallFirst);
   const float inv_n = 1.0f / ((float)n1 * (float)n2);
   // 2D FFT of every plane of x; centred: fftshift(fft2(ifftshift(.)))
   auto fft2 = [&](float2* x, bool inv, bool centred) -> cudaError_t {
@@ -432,30 +645,43 @@ extern "C" odt_status odt_bpm_solve(const odt_bpm_args* a) {
   }
   cmul_plane_kernel<<<g, kThreads, 0, s>>>(fld, pre, plane, nf);
   BPM_CHECK(fft2(fld, true, true));
-  BPM_CHECK(fft2(fld, false, false));
-  // fused march (shared-memory resident planes) for 128 x 128 fields without
-  // the 3D output; ODT_KERNELS=generic keeps the per-slice launches
+  // without the 3D output the slices run fused: in one kernel with the planes
+  // in shared memory for 128 x 128 fields, else in two passes per slice;
+  // ODT_KERNELS=generic keeps the separate launches
   const char* kenv = std::getenv("ODT_KERNELS");
   const bool generic = kenv && std::string(kenv) == "generic";
-  if (n1 == kM && n2 == kM && !out3d && !generic && nz > 0) {
-    BPM_CHECK(cudaFuncSetAttribute(bpm_march128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kMarchSmem));
-    bpm_march128_kernel<<<2 * nill, kMarchThreads, kMarchSmem, s>>>(fld, rk, fm, inv_cos, f1.tw, nz, inv_n);
-    BPM_CHECK(cudaGetLastError());
-  } else {
-  for (int z = 0; z < nz; ++z) {
-    cmul_plane_kernel<<<g, kThreads, 0, s>>>(fld, rk, plane, nf);
-    BPM_CHECK(fft2(fld, true, false));
-    phase_kernel<<<g, kThreads, 0, s>>>(fld, fm + plane * z, inv_cos, plane, nf);
-    BPM_CHECK(fft2(fld, false, false));
-    if (out3d) {
-      fmul_plane_kernel<<<g, kThreads, 0, s>>>(fld, filt, tmp, plane, nf);
-      BPM_CHECK(fft2(tmp, true, false));
-      scatter_slice_kernel<<<g, kThreads, 0, s>>>(tmp, out3d, z, nz, plane, nf);
+  const char* menv = std::getenv("ODT_BPM_MARCH");
+  const bool march = n1 == kM && n2 == kM && !out3d && !generic && !(menv && menv[0] == '0');
+  if (!march && !out3d && !generic && n1 > 1 && n2 > 1) {
+    const long long lines = (long long)n2 * nill;
+    BPM_CHECK(launch_fft_lines(fld, fld, lines, 0, 0, 1.f, false, f1, s));
+    PhaseOp op{fm, inv_cos, 0, n1, n2, inv_n, lines};
+    for (int z = 0; z < nz; ++z, op.fz += plane) {
+      BPM_CHECK(run_cols(fld, rk, n1, nill, f2, s));
+      BPM_CHECK(run_lines(fld, op, fl, z + 1 == nz, s));
     }
+  } else {
+    BPM_CHECK(fft2(fld, false, false));
+    if (march) {
+      BPM_CHECK(cudaFuncSetAttribute(bpm_march128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kMarchSmem));
+      bpm_march128_kernel<<<2 * nill, kMarchThreads, kMarchSmem, s>>>(fld, rk, fm, inv_cos, f1.tw, nz, inv_n);
+      BPM_CHECK(cudaGetLastError());
+    } else {
+      for (int z = 0; z < nz; ++z) {
+        cmul_plane_kernel<<<g, kThreads, 0, s>>>(fld, rk, plane, nf);
+        BPM_CHECK(fft2(fld, true, false));
+        phase_kernel<<<g, kThreads, 0, s>>>(fld, fm + plane * z, inv_cos, plane, nf);
+        BPM_CHECK(fft2(fld, false, false));
+        if (out3d) {
+          fmul_plane_kernel<<<g, kThreads, 0, s>>>(fld, filt, tmp, plane, nf);
+          BPM_CHECK(fft2(tmp, true, false));
+          scatter_slice_kernel<<<g, kThreads, 0, s>>>(tmp, out3d, z, nz, plane, nf);
+        }
+      }
+    }
+    BPM_CHECK(fft2(fld, true, false));
   }
-  }
-  BPM_CHECK(fft2(fld, true, false));
   BPM_CHECK(fft2(fld, false, true));
   cmul_plane_kernel<<<g, kThreads, 0, s>>>(fld, post, plane, nf);
   BPM_CHECK(fft2(fld, true, true));
