@@ -650,8 +650,7 @@ extern "C" odt_status odt_bpm_solve(const odt_bpm_args* a) {
   // ODT_KERNELS=generic keeps the separate launches
   const char* kenv = std::getenv("ODT_KERNELS");
   const bool generic = kenv && std::string(kenv) == "generic";
-  const char* menv = std::getenv("ODT_BPM_MARCH");
-  const bool march = n1 == kM && n2 == kM && !out3d && !generic && !(menv && menv[0] == '0');
+  const bool march = n1 == kM && n2 == kM && !out3d && !generic;
   if (!march && !out3d && !generic && n1 > 1 && n2 > 1) {
     const long long lines = (long long)n2 * nill;
     BPM_CHECK(launch_fft_lines(fld, fld, lines, 0, 0, 1.f, false, f1, s));
