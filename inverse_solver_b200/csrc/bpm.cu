@@ -25,6 +25,7 @@
 
 #include "../../include/odt.h"
 #include "cbs_kernels.cuh"
+#include "pdl.cuh"
 #include "scratch.cuh"
 #include "tile_bodies.cuh"
 
@@ -408,6 +409,8 @@ bpm_lines_kernel(float2* __restrict__ fld, PhaseOp op, const FftPlan plan, const
   const GlobalPlain g{base, base, 1, n, nl};
   const LineMap m{W};
   __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   int ns = 1;   // inverse passes, radices f[P-1] .. f[1]
   for (int i = 0; i + 1 < P; ++i) {
     const int R = plan.radix[P - 1 - i];
@@ -465,6 +468,8 @@ bpm_cols_kernel(float2* __restrict__ fld, const float2* __restrict__ rk, const i
   const ColMap m{lgW};
   const RefocusOp op{rk + i0, n1, ncol};
   __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   int ns = 1;
   for (int p = 0; p + 1 < P; ++p) {   // forward passes f[0] .. f[P-2]
     const int R = plan.radix[p];
@@ -518,8 +523,8 @@ cudaError_t run_lines_c(float2* fld, const PhaseOp& op, const DevFft& f, int las
   const size_t sm = align16(sizeof(float2) * f.plan.n) + 2 * sizeof(float2) * (size_t)W * smem_line_ld(f.plan.n);
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(bpm_lines_kernel<CLS>), sm);
   if (e != cudaSuccess) return e;
-  bpm_lines_kernel<CLS><<<(unsigned)((op.nlines + W - 1) / W), kTileThreads, sm, s>>>(fld, op, f.plan, f.tw, W, last);
-  return cudaGetLastError();
+  return launch_pdl(bpm_lines_kernel<CLS>, 1, (unsigned)((op.nlines + W - 1) / W), kTileThreads, sm, s, fld, op, f.plan,
+                    f.tw, W, last);
 }
 cudaError_t run_lines(float2* fld, const PhaseOp& op, const DevFft& f, int last, cudaStream_t s) {
   BPM_CLS(f, run_lines_c, fld, op, f, last, s)
@@ -531,8 +536,8 @@ cudaError_t run_cols_c(float2* fld, const float2* rk, int n1, int nill, const De
   const size_t sm = align16(sizeof(float2) * f.plan.n) + 2 * sizeof(float2) * (size_t)f.plan.n * (W + 1);
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(bpm_cols_kernel<CLS>), sm);
   if (e != cudaSuccess) return e;
-  bpm_cols_kernel<CLS><<<(unsigned)((n1 + W - 1) / W) * nill, kTileThreads, sm, s>>>(fld, rk, n1, f.plan, f.tw, lg);
-  return cudaGetLastError();
+  return launch_pdl(bpm_cols_kernel<CLS>, 1, (unsigned)((n1 + W - 1) / W) * nill, kTileThreads, sm, s, fld, rk, n1, f.plan,
+                    f.tw, lg);
 }
 cudaError_t run_cols(float2* fld, const float2* rk, int n1, int nill, const DevFft& f, cudaStream_t s) {
   BPM_CLS(f, run_cols_c, fld, rk, n1, nill, f, s)

@@ -12,6 +12,7 @@
 
 #include <string>
 
+#include "prime_pass.cuh"
 #include "scratch.cuh"
 
 namespace odt {
@@ -24,6 +25,7 @@ struct AnyFft {
   const float2* chirp = nullptr;   // [n] exp(-1i pi j^2 / n)
   const float2* bhat_f = nullptr;  // [m] FFT_m(conj(w) wrapped) / m, forward DFT
   const float2* bhat_i = nullptr;  // [m] FFT_m(w wrapped) / m, inverse DFT
+  PrimePlan prime{};               // q != 0: direct products (prime_pass.cu) instead of Bluestein
 };
 
 // Plan for length n on B's stream (tables in B's scratch).

@@ -368,9 +368,11 @@ DevFft make_dev_fft(Handle& H, int n, int kind, const char* what) {
 }
 
 // make_dev_fft for any length: a length with a prime factor above 31 gets a
-// Bluestein plan in *bs (tables on the device, transforms of the 5-smooth
-// length m >= 2 n - 1 through the line / column tiles) and a DevFft with no
-// passes, which no tile kernel accepts.
+// plan in *bs and a DevFft with no passes, which no tile kernel accepts: the
+// direct products of prime_pass.cu where its tables fit shared memory (primes
+// up to about 280), else (and for ODT_KERNELS=generic) Bluestein's algorithm
+// (tables on the device, transforms of the 5-smooth length m >= 2 n - 1
+// through the line / column tiles).
 DevFft make_handle_fft(Handle& H, int n, int kind, const char* what, AnyFft* bs) {
   *bs = AnyFft{};
   bs->n = n;
@@ -378,8 +380,25 @@ DevFft make_handle_fft(Handle& H, int n, int kind, const char* what, AnyFft* bs)
   std::string why;
   if (n < 1) raise(ODT_ERR_INVALID_ARGUMENT, std::string(what) + ": length must be positive");
   if (make_plan(n, &probe, &why, kLargeFirst)) return make_dev_fft(H, n, kind, what);
-  const int m = bluestein_length(n);
   bs->direct = false;
+  DevFft f{};
+  f.plan.n = n;
+  f.plan.npass = 0;
+  PrimePlan pp = H.use_pipe ? prime_plan(n, (size_t)H.max_smem) : PrimePlan{};
+  if (pp.q) {
+    std::vector<float> tab(prime_table_size(pp), 0.f);
+    prime_table(pp, tab.data());
+    const auto tw = make_twiddles(n);
+    float* d_tab = H.dalloc<float>(tab.size(), false);
+    float2* d_tw = H.dalloc<float2>(n, false);
+    ODT_CUDA(cudaMemcpy(d_tab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
+    ODT_CUDA(cudaMemcpy(d_tw, tw.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
+    pp.tab = d_tab;
+    pp.tw = d_tw;
+    bs->prime = pp;
+    return f;
+  }
+  const int m = bluestein_length(n);
   bs->m = m;
   bs->f = make_dev_fft(H, m, kKindCols, what);
   if (fft_smem_bytes(m, bs->f.W, kKindLines) > (size_t)H.max_smem)
@@ -392,9 +411,6 @@ DevFft make_handle_fft(Handle& H, int n, int kind, const char* what, AnyFft* bs)
   bs->chirp = chirp;
   bs->bhat_f = bhat;
   bs->bhat_i = bhat + m;
-  DevFft f{};
-  f.plan.n = n;
-  f.plan.npass = 0;
   return f;
 }
 
@@ -441,8 +457,14 @@ int auto_batch(Handle& H) {
   return (int)nb;
 }
 
+// transform along an axis whose length the radix tiles do not cover
+cudaError_t any_axis(float2* x, int n0, long long n2, bool inv, int sh, float scale, const AnyFft& f, cudaStream_t s) {
+  return f.prime.q ? launch_prime_axis(x, n0, n2, inv, sh, scale, f.prime, s)
+                   : bluestein_axis(x, n0, n2, inv, sh, scale, f, s);
+}
+
 // centred 2D FFT on [n0, n1, nslices] in place (MATLAB fftshift(fft2(ifftshift(x))))
-// (Bluestein on an axis whose length has a prime factor above 31; the
+// (any_axis on an axis whose length has a prime factor above 31; the
 // inverse then normalises axis by axis)
 void fftc2(Handle& H, float2* x, const DevFft& f0, const DevFft& f1, long long nslices,
            bool inverse, cudaStream_t s) {
@@ -459,11 +481,11 @@ void fftc2(Handle& H, float2* x, const DevFft& f0, const DevFft& f1, long long n
     if (b0.direct)
       ODT_CUDA(launch_fft_lines(x, x, (long long)n1 * nslices, n0 / 2, n0 / 2, s0, inverse, f0, s));
     else
-      ODT_CUDA(bluestein_axis(x, 1, (long long)n1 * nslices, inverse, n0 / 2, s0, b0, s));
+      ODT_CUDA(any_axis(x, 1, (long long)n1 * nslices, inverse, n0 / 2, s0, b0, s));
     if (b1.direct)
       ODT_CUDA(launch_fft_cols(x, x, n0, nslices, n1 / 2, n1 / 2, s1, inverse, f1, s));
     else
-      ODT_CUDA(bluestein_axis(x, n0, nslices, inverse, n1 / 2, s1, b1, s));
+      ODT_CUDA(any_axis(x, n0, nslices, inverse, n1 / 2, s1, b1, s));
   }
   H.mark_end(s);
 }
@@ -574,8 +596,13 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   // series of one or two iterations with 1); 16-bit storage and RI tensors
   // go term by term
   const int j0 = B >= 3 && !ten && H.storage != ODT_STORAGE_B16 ? 2 : 1;
-  if (H.any_loop()) {
-    // unfused loop with Bluestein transforms along the uncovered axes
+  // axes the radix tiles do not cover: their transforms run on their own, the
+  // z-pass as one kernel; unfused (products apart from the transforms) where z
+  // has no such kernel and for the generic kernels
+  const bool any_x = !H.bsx.direct, any_y = !H.bsy.direct, any_z = !H.bsz.direct;
+  const bool any = any_z ? !(H.use_pipe && H.bsz.prime.q) : (any_x || any_y) && !H.use_pipe;
+  if (any) {
+    // unfused loop
     if (ten || vec) raise(ODT_ERR_UNSUPPORTED, "RI tensors and dyadic solves need padded lengths whose prime "
                                                "factors are at most 31");
     const long long xl = (long long)a.py * a.pz * nbp, yl = (long long)a.pz * nbp;
@@ -583,16 +610,16 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     auto fft3 = [&](bool inv) {
       auto ax = [&]() {
         if (H.bsx.direct) ODT_CUDA(launch_fft_lines(a.T, a.T, xl, 0, 0, 1.0f, inv, H.fx, s));
-        else ODT_CUDA(bluestein_axis(a.T, 1, xl, inv, 0, 1.0f, H.bsx, s));
+        else ODT_CUDA(any_axis(a.T, 1, xl, inv, 0, 1.0f, H.bsx, s));
       };
       auto ay = [&]() {
         if (H.bsy.direct) ODT_CUDA(launch_fft_cols(a.T, a.T, a.px, yl, 0, 0, 1.0f, inv, H.fy, s));
-        else ODT_CUDA(bluestein_axis(a.T, a.px, yl, inv, 0, 1.0f, H.bsy, s));
+        else ODT_CUDA(any_axis(a.T, a.px, yl, inv, 0, 1.0f, H.bsy, s));
       };
       auto az = [&]() {
         if (pxy > INT32_MAX) raise(ODT_ERR_UNSUPPORTED, "x-y plane too large for the column transforms");
         if (H.bsz.direct) ODT_CUDA(launch_fft_cols(a.T, a.T, (int)pxy, nbp, 0, 0, 1.0f, inv, H.fz, s));
-        else ODT_CUDA(bluestein_axis(a.T, (int)pxy, nbp, inv, 0, 1.0f, H.bsz, s));
+        else ODT_CUDA(any_axis(a.T, (int)pxy, nbp, inv, 0, 1.0f, H.bsz, s));
       };
       H.mark_begin(kKBornY, s);
       if (inv) { az(); ay(); ax(); } else { ax(); ay(); az(); }
@@ -613,12 +640,11 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     ODT_CUDA(launch_born_point(a, kBornLast, B + 1, s));
     H.mark_end(s);
   }
-  const bool any = H.any_loop();
-  const bool pipe_x = !any && !ten && H.use_pipe && born_x_pipe_supported(a, H.fx);
-  const bool pipe_y = !any && H.use_pipe && cols_pipe_supported(a, H.fy, false);
+  const bool pipe_x = !any && !any_x && !ten && H.use_pipe && born_x_pipe_supported(a, H.fx);
+  const bool pipe_y = !any && !any_y && H.use_pipe && cols_pipe_supported(a, H.fy, false);
   // 16-bit storage keeps its own z-pass (set up below); the others share one
   const bool b16 = H.storage == ODT_STORAGE_B16;
-  const bool pipe_z = !any && !vec && H.use_pipe &&
+  const bool pipe_z = !any && !any_z && !vec && H.use_pipe &&
                       (b16 ? cols_pipe_supported(a, H.fz, true) : z_pass_supported(a, H.fz));
   // (reported as born_z_pipe on 8 R points, R of the 16-bit pass; as born_z elsewhere)
   const int zkind = pipe_z && cols_pipe_supported(a, H.fz, true) ? kKBornZPipe : kKBornZ;
@@ -630,7 +656,7 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   const long long xlines = (long long)a.py * a.pz * nbp;
   // fused xy-pass (x- and both y-passes in one kernel; the z-pass, pipelined,
   // dyadic or generic, reads its permuted x-y spectrum): scalar potentials
-  const bool fused_xy = !any && !ten && H.use_pipe && H.use_xy && B >= 1 && born_xy_supported(a, H.max_smem, b16);
+  const bool fused_xy = !any && !any_x && !any_y && !ten && H.use_pipe && H.use_xy && B >= 1 && born_xy_supported(a, H.max_smem, b16);
   a.perm_xy = fused_xy ? 1 : 0;
   if (b16) {
     if (!fused_xy || !pipe_z)
@@ -657,7 +683,9 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     ODT_CUDA(launch_born_xy(a, jj == j0 ? kBornFirst : kBornMid, jj, H.fx, s));
     H.mark_end(s);
     H.mark_begin(zkind, s);
-    if (vec)
+    if (any_z)
+      ODT_CUDA(launch_prime_z(a, jj, H.bsz.prime, s));
+    else if (vec)
       ODT_CUDA(launch_born_z_dyadic(a, dy, jj, H.fz, H.max_smem, s));
     else if (pipe_z && b16)
       ODT_CUDA(launch_born_z_pipe(a, jj, H.fz, H.d_fault, s));
@@ -678,6 +706,11 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
       if (jj >= 2) ODT_CUDA(launch_fft_lines(a.T, a.T, xlines, 0, 0, 1.0f, true, H.fx, s));
       ODT_CUDA(launch_born_tensor_point(a, P.V9, jj == 1 ? kBornFirst : kBornMid, jj, s));
       ODT_CUDA(launch_fft_lines(a.T, a.T, xlines, 0, 0, 1.0f, false, H.fx, s));
+    } else if (any_x) {
+      H.mark_begin(kKBornX, s);
+      if (jj > j0) ODT_CUDA(any_axis(a.T, 1, xlines, true, 0, 1.0f, H.bsx, s));
+      ODT_CUDA(launch_born_point(a, jj == j0 ? kBornFirst : kBornMid, jj, s));
+      ODT_CUDA(any_axis(a.T, 1, xlines, false, 0, 1.0f, H.bsx, s));
     } else if (pipe_x && jj > j0) {
       H.mark_begin(kKBornXPipe, s);
       ODT_CUDA(launch_born_x_pipe(a, kBornMid, jj, H.fx, H.d_fault, s));
@@ -687,13 +720,17 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     }
     H.mark_end(s);
     H.mark_begin(pipe_y ? kKBornYPipe : kKBornY, s);
-    if (pipe_y)
+    if (any_y)
+      ODT_CUDA(any_axis(a.T, a.px, (long long)a.pz * nbp, false, 0, 1.0f, H.bsy, s));
+    else if (pipe_y)
       ODT_CUDA(launch_fft_y_pipe(a, false, H.fy, H.d_fault, s));
     else
       ODT_CUDA(launch_fft_cols(a.T, a.T, a.px, (long long)a.pz * nbp, 0, 0, 1.0f, false, H.fy, s));
     H.mark_end(s);
     H.mark_begin(zkind, s);
-    if (vec)
+    if (any_z)
+      ODT_CUDA(launch_prime_z(a, jj, H.bsz.prime, s));
+    else if (vec)
       ODT_CUDA(launch_born_z_dyadic(a, dy, jj, H.fz, H.max_smem, s));
     else if (pipe_z)
       ODT_CUDA(launch_z_pass(a, jj, H.fz, H.d_fault, s));
@@ -701,7 +738,9 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
       ODT_CUDA(launch_born_z(a, jj, H.fz, s));
     H.mark_end(s);
     H.mark_begin(pipe_y ? kKBornYPipe : kKBornY, s);
-    if (pipe_y)
+    if (any_y)
+      ODT_CUDA(any_axis(a.T, a.px, (long long)a.pz * nbp, true, 0, 1.0f, H.bsy, s));
+    else if (pipe_y)
       ODT_CUDA(launch_fft_y_pipe(a, true, H.fy, H.d_fault, s));
     else
       ODT_CUDA(launch_fft_cols(a.T, a.T, a.px, (long long)a.pz * nbp, 0, 0, 1.0f, true, H.fy, s));
@@ -712,6 +751,10 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
       H.mark_begin(kKBornX, s);
       if (B >= 1) ODT_CUDA(launch_fft_lines(a.T, a.T, xlines, 0, 0, 1.0f, true, H.fx, s));
       ODT_CUDA(launch_born_tensor_point(a, P.V9, kBornLast, B + 1, s));
+    } else if (any_x) {
+      H.mark_begin(kKBornX, s);
+      if (B >= 1) ODT_CUDA(any_axis(a.T, 1, xlines, true, 0, 1.0f, H.bsx, s));
+      ODT_CUDA(launch_born_point(a, kBornLast, B + 1, s));
     } else if (pipe_x && B + 1 >= 2) {
       H.mark_begin(kKBornXPipeEdge, s);
       ODT_CUDA(launch_born_x_pipe(a, kBornLast, B + 1, H.fx, H.d_fault, s));
@@ -1523,7 +1566,7 @@ odt_status odt_autotune(odt_handle h, int32_t n_ill, odt_tune_result* out) {
     probe.py = H->g.sim_size[1];
     probe.pz = H->g.sim_size[2];
     probe.nbatch = nb * H->np;
-    const bool xy_ok = !H->pot[0].tensor && !H->any_loop() &&
+    const bool xy_ok = !H->pot[0].tensor && H->bsx.direct && H->bsy.direct &&
                        born_xy_supported(probe, H->max_smem, H->storage == ODT_STORAGE_B16);
     const bool saved_xy = H->use_xy, saved_pipe = H->use_pipe;
     const bool want_t = H->ktrans != nullptr;

@@ -14,10 +14,8 @@
 
 namespace odt {
 
-#if defined(__CUDA_ARCH__)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-#endif
 
 template <class... P, class... A>
 cudaError_t launch_pdl(void (*kernel)(P...), int cluster, unsigned grid, unsigned block, size_t smem, cudaStream_t s,
