@@ -48,17 +48,10 @@
 // CTA barriers (after steps 1 and 6), and the warps drift apart so that one
 // warp's global loads overlap other warps' transforms.
 //
-// Bank conflicts: rows have a pitch of N = 8 (mod 16) complex elements for
-// odd R.  Steps 1, 2, 6, 7 put consecutive x on consecutive lanes; steps 3
-// and 5 take R consecutive elements at R k1 (lanes over k1 and rows: the
-// stride of 2R banks and the row pitch of 16 banks keep a half-warp's 8-byte
-// accesses on distinct bank pairs); step 4 takes consecutive n2 on
-// consecutive lanes.  For even R (N = 96, 128) a stride of R elements puts
-// several k1 on the same banks (all eight at R = 16), so those planes carry
-// one pad element after every R elements of a row (XYSmem::sx): group k1
-// starts at (R + 1) k1, eight distinct bank pairs, and the pitch N + N / R
-// is 8 (mod 16); the four rows of a warp's step-3 / -5 access still share
-// banks (two wavefronts where one would do).
+// Bank conflicts: steps 1, 2, 6, 7 put consecutive x on consecutive lanes;
+// steps 3 and 5 take R consecutive elements at R k1 (lanes over k1 and rows),
+// step 4 consecutive n2 on consecutive lanes.  XYSmem::sx and the row pitch
+// keep a half-warp's 8-byte accesses of steps 3 and 5 on distinct bank pairs.
 #include <cuda_runtime.h>
 
 #include "b16.cuh"
@@ -88,6 +81,16 @@ constexpr size_t a128(size_t b) { return (b + 127) & ~(size_t)127; }
 constexpr int kMaxR16 = 20;   // largest R of the 16-bit storage
 constexpr int xy_ctas(int r) { return r > 20 || (r >= 14 && r % 2 == 0) ? 2 : 1; }
 
+// smallest row pitch with pitch * h = 8 (mod 16) elements whose buffer lets
+// `per_sm` CTAs of `tables` bytes more share an SM (227 KB, 1 KB a CTA
+// reserved); the unpadded one if there is none
+constexpr int xy_pitch(int r, int h, size_t tables, int per_sm) {
+  const int p0 = 8 * r + (r % 2 == 0 ? 8 : 0);
+  for (int p = p0; p < p0 + 16; ++p)
+    if (p * h % 16 == 8 && tables + sizeof(float2) * 8 * h * p <= (size_t)227 * 1024 / per_sm - 1024) return p;
+  return p0;
+}
+
 template <int R>
 struct XYSmem {
   static constexpr int C = xy_ctas(R);
@@ -103,12 +106,13 @@ struct XYSmem {
   static constexpr int kTkS = R | 1;
   static constexpr size_t kTk = kMaskY + a16(sizeof(float) * N);
   static constexpr size_t kPlane = a128(kTk + a16(sizeof(float2) * 8 * kTkS));
-  // plane rows: for odd R a pitch of N (= 8 mod 16) elements; for even R
-  // (N = 96, 128: 0 mod 16) one pad element after every R elements of a row,
-  // so that the groups R k1 .. R k1 + R-1 of steps 3 and 5 start on
-  // different banks ((R + 1) k1) and the pitch N + N / R is 8 mod 16 again
+  // plane rows: for even R one pad element after every R elements, so that the
+  // groups R k1 .. R k1 + R-1 of steps 3 and 5 start on different banks; the
+  // pitch P makes H rows a shift of 8 (mod 16) elements, so that the two rows
+  // a half-warp takes there fill the other half of the banks (27 = 8 * 14
+  // rows: P = 220 instead of 216, where both rows met on the same banks)
   static constexpr bool kPad = R % 2 == 0;
-  static constexpr int P = kPad ? N + N / R : N;
+  static constexpr int P = xy_pitch(R, H, kPlane, C == 2 && R <= 20 ? 2 : 1);
   static constexpr size_t kTotal = kPlane + sizeof(float2) * 8 * H * P;
   // in-row position of x
   static __device__ __forceinline__ int sx(int x) { return kPad ? x + x / R : x; }
