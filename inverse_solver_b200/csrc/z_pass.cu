@@ -3,10 +3,10 @@
 // z-FFT (FORWARD_SOLVER_CONVERGENT_BORN.m:606-615), the same transforms as
 // born_z_body.
 //
-//   * persistent CTAs walk tiles of 16 adjacent columns of the flattened x-y
+//   * persistent CTAs walk tiles of 16 or 32 adjacent columns of the flattened x-y
 //     plane (so a plane wastes at most one partial tile: 152 columns in rows
 //     of their own would fill 9.5 of 10 tiles);
-//   * a tile (n rows of 128 bytes) arrives in shared memory while the CTA
+//   * a tile (n rows of 128 or 256 bytes) arrives in shared memory while the CTA
 //     computes the previous one from the other stage: through one tiled TMA
 //     copy on an mbarrier where the planes are multiples of 16 bytes (px * py
 //     even), else through 8-byte asynchronous copies of the threads;
@@ -37,7 +37,10 @@
 namespace odt {
 namespace {
 
-constexpr int kW = 16;          // columns per tile
+// columns per tile: 16; 32 for A <= 5, where step B would keep only 16 A of the
+// threads busy (85 = 5 x 17 points behind an 88 x 88 plane, 8
+// illuminations: 39.9 -> 33.3 us; 69 = 3 x 23, 125 x 108 plane: 53 -> 40 us)
+__host__ __device__ constexpr int tile_w(int A) { return A <= 5 ? 32 : 16; }
 constexpr int kThreads = 160;
 constexpr int kMaxN = 256;      // rows of a TMA box
 constexpr int kMaxR = 31;
@@ -72,13 +75,13 @@ __host__ __device__ constexpr size_t a1k(size_t b) { return (b + 1023) & ~(size_
 // two landing stages on 1024-byte boundaries (tiled copies need 128)
 struct ZSmem {
   size_t tw, kz, gxy, s0, s1, total;
-  __host__ __device__ explicit ZSmem(int n) {
+  __host__ __device__ ZSmem(int n, int w) {
     tw = 64;
     kz = tw + a16(sizeof(float2) * n);
     gxy = kz + a16(sizeof(float) * n);
-    s0 = a1k(gxy + a16(sizeof(float) * kW));
-    s1 = s0 + sizeof(float2) * n * kW;
-    total = s1 + sizeof(float2) * n * kW;
+    s0 = a1k(gxy + a16(sizeof(float) * w));
+    s1 = s0 + sizeof(float2) * n * w;
+    total = s1 + sizeof(float2) * n * w;
   }
 };
 
@@ -115,7 +118,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
                   int* __restrict__ fault) {
 #if defined(__CUDA_ARCH__)
   const int N = A_ * R;
-  const ZSmem L(N);
+  const int W = kEight ? 16 : tile_w(A_);
+  const ZSmem L(N, W);
   extern __shared__ __align__(128) unsigned char sm[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
   float2* tw = reinterpret_cast<float2*>(sm + L.tw);
@@ -124,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
   float2* const s0 = reinterpret_cast<float2*>(sm + L.s0);
   float2* const s1 = reinterpret_cast<float2*>(sm + L.s1);
   const int tid = threadIdx.x;
-  const int c = tid & (kW - 1);
+  const int c = tid & (W - 1);
   const bool flip = a.acyclic && (jj & 1);
   if ((smem_addr(s0) & 127u) != 0u || (smem_addr(s1) & 127u) != 0u) {  // never issue a misaligned copy
     if (tid == 0) atomicCAS(fault, 0, kFaultAlign);
@@ -143,11 +147,11 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
   int tile = blockIdx.x;
   if (tile >= ntiles) return;
   const int pxy = a.px * a.py;            // row stride of a column
-  const uint32_t bytes = (uint32_t)(sizeof(float2) * N * kW);
-  // tile t -> (16 columns from i0 = 16 (t mod nxt), batch entry t / nxt)
+  const uint32_t bytes = (uint32_t)(sizeof(float2) * N * W);
+  // tile t -> (W columns from i0 = W (t mod nxt), batch entry t / nxt)
   auto issue = [&](int t, int stage) {
     float2* dst = stage ? s1 : s0;
-    const int i0 = kW * (t % nxt), b = t / nxt;
+    const int i0 = W * (t % nxt), b = t / nxt;
     if (use_tma) {
       if (tid == 0) {
         fence_proxy_async();
@@ -157,7 +161,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
     } else {
       const int col = min(i0 + c, pxy - 1);   // columns past the plane repeat the last one; not stored
       const float2* src = a.T + (long long)b * a.nvox + col;
-      for (int r = tid >> 4; r < N; r += kThreads / kW) copy8(dst + r * kW + c, src + (long long)r * pxy);
+      for (int r = tid / W; r < N; r += kThreads / W) copy8(dst + r * W + c, src + (long long)r * pxy);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
   };
@@ -168,8 +172,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
     const int s = it & 1;
     const int next = tile + gridDim.x;
     if (next < ntiles) issue(next, s ^ 1);
-    const int i0 = kW * (tile % nxt), b = tile / nxt;
-    if (tid < kW) {
+    const int i0 = W * (tile % nxt), b = tile / nxt;
+    if (tid < W) {
       const int i = min(i0 + tid, pxy - 1);
       int y = i / a.px, kx = i - y * a.px;
       if (a.perm_xy) {   // position Rx k1 + k2 holds spectral index k1 + 8 k2
@@ -205,8 +209,9 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
       constexpr int A = decltype(Ac)::value;
       if constexpr (ZSplit<A * R>::kA == A && (A == 8) == kEight) {
         constexpr int kN = A * R;
+        constexpr int kW = tile_w(A);
         // ---- A: A-point DFT over n1 at rows R n1 + n2, times W_N^(n2 k1)
-        for (int n2 = tid >> 4; n2 < R; n2 += kThreads / kW) {
+        for (int n2 = tid / kW; n2 < R; n2 += kThreads / kW) {
           float2 v[A];
 #pragma unroll
           for (int r = 0; r < A; ++r) v[r] = S[(R * r + n2) * kW + c];
@@ -239,13 +244,13 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
           for (int r = 0; r < R; ++r) S[(R * k1 + r) * kW + c] = v[r];
         };
         if constexpr (A <= kThreads / kW) {   // one round
-          if (tid < A * kW) mid(tid >> 4);
+          if (tid < A * kW) mid(tid / kW);
         } else {
-          for (int k1 = tid >> 4; k1 < A; k1 += kThreads / kW) mid(k1);
+          for (int k1 = tid / kW; k1 < A; k1 += kThreads / kW) mid(k1);
         }
         __syncthreads();
         // ---- C: inverse A-point DFT over k1 -> rows R n1 + n2 of T
-        for (int n2 = tid >> 4; n2 < R; n2 += kThreads / kW) {
+        for (int n2 = tid / kW; n2 < R; n2 += kThreads / kW) {
           float2 v[A];
 #pragma unroll
           for (int r = 0; r < A; ++r) v[r] = S[(R * r + n2) * kW + c];
@@ -285,15 +290,15 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
   return fn;
 }
 
-// T viewed as float32 pairs: dims (inner first) {2 px py, pz, nb}, box 32
-// floats = 16 complex columns by all rows
-bool make_map(const BornArgs& a, CUtensorMap* m) {
+// T viewed as float32 pairs: dims (inner first) {2 px py, pz, nb}, box 2 W
+// floats = W complex columns by all rows
+bool make_map(const BornArgs& a, int W, CUtensorMap* m) {
   auto enc = encoder();
   if (!enc) return false;
   const cuuint64_t plane = (cuuint64_t)a.px * a.py;
   const cuuint64_t dims[3] = {2 * plane, (cuuint64_t)a.pz, (cuuint64_t)a.nbatch};
   const cuuint64_t strides[2] = {plane * sizeof(float2), plane * sizeof(float2) * a.pz};
-  const cuuint32_t box[3] = {2 * kW, (cuuint32_t)a.pz, 1};
+  const cuuint32_t box[3] = {2 * (cuuint32_t)W, (cuuint32_t)a.pz, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, a.T, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -302,7 +307,8 @@ bool make_map(const BornArgs& a, CUtensorMap* m) {
 
 template <int R, bool kEight>
 cudaError_t launch_one(const BornArgs& a, int jj, const DevFft& f, int* fault, cudaStream_t s) {
-  const ZSmem L(a.pz);
+  const int W = tile_w(a.pz / R);
+  const ZSmem L(a.pz, W);
   const void* fn = reinterpret_cast<const void*>(z_pass_kernel<R, kEight>);
   cudaError_t e = raise_smem_limit(fn, L.total);
   if (e != cudaSuccess) return e;
@@ -315,8 +321,8 @@ cudaError_t launch_one(const BornArgs& a, int jj, const DevFft& f, int* fault, c
   CUtensorMap map{};
   // planes that are no multiple of 16 bytes cannot be mapped: 8-byte copies
   const int use_tma = (long long)a.px * a.py % 2 == 0;
-  if (use_tma && !make_map(a, &map)) return cudaErrorInvalidValue;
-  const int nxt = (a.px * a.py + kW - 1) / kW;
+  if (use_tma && !make_map(a, W, &map)) return cudaErrorInvalidValue;
+  const int nxt = (a.px * a.py + W - 1) / W;
   const int ntiles = nxt * a.nbatch;
   const int cap = per_sm * nsm;
   z_pass_kernel<R, kEight><<<ntiles < cap ? ntiles : cap, kThreads, L.total, s>>>(map, a, jj, f.tw, a.pz / R, use_tma, nxt,
@@ -358,7 +364,7 @@ ODT_Z_HERE(13) ODT_Z_HERE(27) ODT_Z_HERE(30) ODT_Z_HERE(10) ODT_Z_HERE(7)
 bool z_pass_supported(const BornArgs& a, const DevFft& f) {
   if (f.plan.n != a.pz || a.pz > kMaxN || a.storage || !z_split(a.pz) || !encoder()) return false;
   const long long pxy = (long long)a.px * a.py;
-  return pxy < (1 << 30) && (pxy + kW - 1) / kW * a.nbatch < (1LL << 31);
+  return pxy < (1 << 30) && (pxy + 15) / 16 * a.nbatch < (1LL << 31);
 }
 
 cudaError_t launch_z_pass(const BornArgs& a, int jj, const DevFft& fz, int* fault, cudaStream_t s) {
