@@ -445,8 +445,11 @@ void ensure_batch(Handle& H, int nb) {
   H.batch = nb;
 }
 
-int auto_batch(Handle& H) {
+// illuminations per batch for a call of n: buffers that already hold n need no
+// look at the free memory (a driver query of tens of microseconds per solve)
+int auto_batch(Handle& H, int n) {
   if (H.g.max_batch > 0) return H.g.max_batch;
+  if (H.batch >= n) return H.batch;
   size_t free_b = 0, total_b = 0;
   ODT_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const size_t held = H.static_bytes;  // batch buffers are reallocated, not added
@@ -1167,7 +1170,7 @@ odt_status odt_solve(odt_handle h, const odt_solve_args* args) {
     }
     // device pointers: the caller's stream as given (NULL = legacy default stream)
     cudaStream_t s = dev ? (cudaStream_t)A.stream : H->own_stream;
-    const int want_batch = std::min<int>(A.n_ill, auto_batch(*H));
+    const int want_batch = std::min<int>(A.n_ill, auto_batch(*H, A.n_ill));
     ensure_batch(*H, want_batch);
     const cudaMemcpyKind kin = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const cudaMemcpyKind kout = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
@@ -1224,7 +1227,7 @@ odt_status odt_solve_source(odt_handle h, const odt_source_args* args) {
     if (dev && (!is_device_ptr(A.source) || !is_device_ptr(A.field3d)))
       raise(ODT_ERR_INVALID_ARGUMENT, "odt_solve_source: ODT_MEM_DEVICE with a non-device pointer");
     cudaStream_t s = dev ? (cudaStream_t)A.stream : H->own_stream;
-    ensure_batch(*H, std::min<int>(A.n, auto_batch(*H)));
+    ensure_batch(*H, std::min<int>(A.n, auto_batch(*H, A.n)));
     const cudaMemcpyKind kin = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const cudaMemcpyKind kout = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     const long long nR = H->nri() * H->np;   // complex values per source / field
@@ -1267,7 +1270,7 @@ odt_status odt_gradient(odt_handle h, const odt_gradient_args* args) {
                 !is_device_ptr(A.grad)))
       raise(ODT_ERR_INVALID_ARGUMENT, "odt_gradient: ODT_MEM_DEVICE with a non-device pointer");
     cudaStream_t s = dev ? (cudaStream_t)A.stream : H->own_stream;
-    ensure_batch(*H, std::min<int>(A.n_ill, auto_batch(*H)));
+    ensure_batch(*H, std::min<int>(A.n_ill, auto_batch(*H, A.n_ill)));
     // per illumination: npol planes of [F_x, F_y] in, np components of [ri] in 3D;
     // the gradient is the mean over components and illuminations (the
     // reference's mean(..., [4 5]) over [ri, pole_num, n_ill])
@@ -1541,7 +1544,7 @@ odt_status odt_autotune(odt_handle h, int32_t n_ill, odt_tune_result* out) {
     if (!H->pot[0].have) raise(ODT_ERR_NOT_READY, "odt_autotune: call odt_set_potential first");
     if (H->np == 3 && !H->have_pol) raise(ODT_ERR_NOT_READY, "odt_autotune: set the polarisation basis first");
     DeviceGuard dg(H->g.device);
-    const int nb = std::min<int>(n_ill, auto_batch(*H));
+    const int nb = std::min<int>(n_ill, auto_batch(*H, n_ill));
     ensure_batch(*H, nb);
     const TuneKey key{H->g.device, H->g.sim_size[0], H->g.sim_size[1], H->g.sim_size[2], nb, H->np, H->storage};
     {

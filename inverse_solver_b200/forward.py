@@ -187,17 +187,21 @@ class CBSHostSetup:
         self.tensor = True
         return pp, keep + [_c64(V)]
 
-    def potential_params(self, eps_imag):
-        """The RI-independent part of create_boundary_RI and init
-        (FORWARD_SOLVER_CONVERGENT_BORN.m:251-396) for a given eps_imag:
-        attenuation masks, ramps, Green's coordinates, Bornmax and the
-        scalars, as the PotentialParams struct plus the arrays it points
-        into (keep them alive until the call returns)."""
+    def _potential_tables(self):
+        """The tables of create_boundary_RI and init
+        (FORWARD_SOLVER_CONVERGENT_BORN.m:251-396) that depend on neither the
+        RI nor eps_imag: attenuation masks, ramps, Green's coordinates, optical
+        tool of the padded grid.  Built once per set of the parameters they
+        read (an outer loop sets two potentials per iteration; building them
+        each time took about 1 ms of each on a 64 x 64 x 61 grid)."""
         p = self.parameters
-        self.eps_imag = F32(eps_imag)
         btp = [int(b) for b in self.boundary_thickness_pixel]
+        key = (tuple(btp), tuple(self.expected_RI_size), bool(self.cyclic_boundary_xy), bool(p["acyclic"]),
+               float(p["boundary_sharpness"]), tuple(float(r) for r in p["resolution"]), float(p["wavelength"]),
+               float(p["NA"]), float(p["RI_bg"]))
+        if getattr(self, "_tables_key", None) == key:
+            return self._tables
         old = list(self.expected_RI_size)
-        self.ROI = [btp[0] + 1, btp[0] + old[0], btp[1] + 1, btp[1] + old[1], btp[2] + 1, btp[2] + old[2]]
         shape = tuple(old[j] + 2 * btp[j] for j in range(3))
         masks = []
         for j in range(3):
@@ -216,7 +220,7 @@ class CBSHostSetup:
         # init :280-396
         pb = copy.deepcopy(p)
         pb["size"] = list(shape)
-        ub = self.utility_border = OpticalTool(pb)
+        ub = OpticalTool(pb)
         if p["acyclic"] and self.cyclic_boundary_xy:
             sc = [ub.fourier_coor[0], ub.fourier_coor[1], ub.fourier_coor[2] + ub.fourier_res[2] / 4]
         elif p["acyclic"]:
@@ -225,15 +229,8 @@ class CBSHostSetup:
             sc = list(ub.fourier_coor)
         kq2 = [np.fft.ifftshift(c * c).astype(F32) for c in sc]
         # dyadic Green's function: rads = shifted coordinate / k0_nm (:316-319),
-        # ifftshifted (:385), and the absorptive correction (:322)
+        # ifftshifted (:385)
         rads = [np.fft.ifftshift((np.asarray(c, dtype=F32) / ub.k0_nm).astype(F32)) for c in sc]
-        a2 = F32((2 * math.pi * ub.k0_nm) ** 2)
-        absorb = C64(a2 / C64(a2 + 1j * self.eps_imag))
-        step = F32(abs(2 * (2 * math.pi * ub.k0_nm) / self.eps_imag))
-        nrm = float(np.linalg.norm(np.asarray(shape, dtype=np.float64) * np.asarray(p["resolution"], dtype=np.float64)))
-        bopt = int(math.ceil(float(F32(F32(nrm / step) / 2 + 1)))) * 2
-        it = p["iterations_number"]
-        self.Bornmax = 0 if it == 0 else (bopt * abs(int(it)) if it < 0 else int(it))
         ramps = []
         if p["acyclic"]:
             for j in range(3):
@@ -249,6 +246,31 @@ class CBSHostSetup:
                     ramps.append(x / x[n // 2])
         else:
             ramps = [np.ones(shape[j], dtype=C64) for j in range(3)]
+        self._tables = (shape, ub, masks, ramps, kq2, rads)
+        self._tables_key = key
+        return self._tables
+
+    def potential_params(self, eps_imag):
+        """The RI-independent part of create_boundary_RI and init
+        (FORWARD_SOLVER_CONVERGENT_BORN.m:251-396) for a given eps_imag:
+        attenuation masks, ramps, Green's coordinates, Bornmax and the
+        scalars, as the PotentialParams struct plus the arrays it points
+        into (keep them alive until the call returns)."""
+        p = self.parameters
+        self.eps_imag = F32(eps_imag)
+        btp = [int(b) for b in self.boundary_thickness_pixel]
+        old = list(self.expected_RI_size)
+        self.ROI = [btp[0] + 1, btp[0] + old[0], btp[1] + 1, btp[1] + old[1], btp[2] + 1, btp[2] + old[2]]
+        shape, ub, masks, ramps, kq2, rads = self._potential_tables()
+        self.utility_border = ub
+        # the absorptive correction of the dyadic Green's function (:322)
+        a2 = F32((2 * math.pi * ub.k0_nm) ** 2)
+        absorb = C64(a2 / C64(a2 + 1j * self.eps_imag))
+        step = F32(abs(2 * (2 * math.pi * ub.k0_nm) / self.eps_imag))
+        nrm = float(np.linalg.norm(np.asarray(shape, dtype=np.float64) * np.asarray(p["resolution"], dtype=np.float64)))
+        bopt = int(math.ceil(float(F32(F32(nrm / step) / 2 + 1)))) * 2
+        it = p["iterations_number"]
+        self.Bornmax = 0 if it == 0 else (bopt * abs(int(it)) if it < 0 else int(it))
         pp = _lib.PotentialParams()
         pp.eps_imag = float(self.eps_imag)
         pp.green_scale = float(F32(4 * math.pi ** 2))
@@ -265,11 +287,12 @@ class CBSHostSetup:
             pp.kq2[j] = _lib.ptr(keep[6 + j])
             pp.rad[j] = _lib.ptr(keep[9 + j])
         pp.absorb[:] = [float(absorb.real), float(absorb.imag)]
-        self.rads1d = rads
+        # copies: these attributes are the caller's to change, the tables are not
+        self.rads1d = [r.copy() for r in rads]
         self.green_absorbtion_correction = absorb
-        self.attenuation_mask1d = masks
-        self.ramp1d = ramps
-        self.kq2 = kq2
+        self.attenuation_mask1d = [m.copy() for m in masks]
+        self.ramp1d = [r.copy() for r in ramps]
+        self.kq2 = [k.copy() for k in kq2]
         return pp, keep
 
     def voxel_iterations(self, n_ill):
