@@ -129,6 +129,10 @@ cudaError_t launch_born_z_pipe(const BornArgs& a, int jj, const DevFft& fz, int*
 // storage; same results as launch_born_z up to the order of the FFT arithmetic.
 bool z_pass_supported(const BornArgs& a, const DevFft& f);
 cudaError_t launch_z_pass(const BornArgs& a, int jj, const DevFft& fz, int* fault, cudaStream_t s);
+// Pipelined y-FFT in place on a.T for the same lengths (y_pass.cu); same
+// results as launch_fft_cols up to the order of the FFT arithmetic.
+bool y_pass_supported(const BornArgs& a, const DevFft& f);
+cudaError_t launch_y_pass(const BornArgs& a, bool inverse, const DevFft& fy, int* fault, cudaStream_t s);
 // Fused xy-pass (born_xy.cu): the whole x-y plane of one z and illumination
 // in shared memory -- inverse y- and x-FFT of T, update of iteration jj-1,
 // source of iteration jj, forward x- and y-FFT -- for px == py = 8 * {11, 12,

@@ -645,6 +645,7 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   }
   const bool pipe_x = !any && !any_x && !ten && H.use_pipe && born_x_pipe_supported(a, H.fx);
   const bool pipe_y = !any && !any_y && H.use_pipe && cols_pipe_supported(a, H.fy, false);
+  const bool any_len_y = !any && !any_y && !pipe_y && H.use_pipe && y_pass_supported(a, H.fy);
   // 16-bit storage keeps its own z-pass (set up below); the others share one
   const bool b16 = H.storage == ODT_STORAGE_B16;
   const bool pipe_z = !any && !any_z && !vec && H.use_pipe &&
@@ -727,6 +728,8 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
       ODT_CUDA(any_axis(a.T, a.px, (long long)a.pz * nbp, false, 0, 1.0f, H.bsy, s));
     else if (pipe_y)
       ODT_CUDA(launch_fft_y_pipe(a, false, H.fy, H.d_fault, s));
+    else if (any_len_y)
+      ODT_CUDA(launch_y_pass(a, false, H.fy, H.d_fault, s));
     else
       ODT_CUDA(launch_fft_cols(a.T, a.T, a.px, (long long)a.pz * nbp, 0, 0, 1.0f, false, H.fy, s));
     H.mark_end(s);
@@ -745,6 +748,8 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
       ODT_CUDA(any_axis(a.T, a.px, (long long)a.pz * nbp, true, 0, 1.0f, H.bsy, s));
     else if (pipe_y)
       ODT_CUDA(launch_fft_y_pipe(a, true, H.fy, H.d_fault, s));
+    else if (any_len_y)
+      ODT_CUDA(launch_y_pass(a, true, H.fy, H.d_fault, s));
     else
       ODT_CUDA(launch_fft_cols(a.T, a.T, a.px, (long long)a.pz * nbp, 0, 0, 1.0f, true, H.fy, s));
     H.mark_end(s);
