@@ -99,6 +99,9 @@ cudaError_t launch_pol32(const float2* in, float2* out, const PolTables& t, bool
 // z-pass with the dyadic Green's function; a.nbatch = 3 * illuminations
 cudaError_t launch_born_z_dyadic(const BornArgs& a, const DyadArgs& d, int jj, const DevFft& fz,
                                  int max_smem, cudaStream_t s);
+// the same for z lengths A R <= 256 (z_dyadic.cu)
+bool z_dyadic_supported(const BornArgs& a, const DevFft& f, int max_smem);
+cudaError_t launch_z_dyadic(const BornArgs& a, const DyadArgs& d, int jj, const DevFft& fz, cudaStream_t s);
 // RI tensor (V9 [nvox, 3, 3]): the x-pass's pointwise work of iteration jj
 // (mode First / Mid / Last as launch_born_x) on the inverse x-FFT in a.T, and
 // the output stage's emitter into conv [c0, c1, rz, a.nbatch]

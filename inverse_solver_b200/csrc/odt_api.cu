@@ -645,6 +645,7 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
   }
   const bool pipe_x = !any && !any_x && !ten && H.use_pipe && born_x_pipe_supported(a, H.fx);
   const bool pipe_y = !any && !any_y && H.use_pipe && cols_pipe_supported(a, H.fy, false);
+  const bool pipe_zd = vec && H.use_pipe && z_dyadic_supported(a, H.fz, H.max_smem);
   const bool any_len_y = !any && !any_y && !pipe_y && H.use_pipe && y_pass_supported(a, H.fy);
   // 16-bit storage keeps its own z-pass (set up below); the others share one
   const bool b16 = H.storage == ODT_STORAGE_B16;
@@ -689,6 +690,8 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     H.mark_begin(zkind, s);
     if (any_z)
       ODT_CUDA(launch_prime_z(a, jj, H.bsz.prime, s));
+    else if (pipe_zd)
+      ODT_CUDA(launch_z_dyadic(a, dy, jj, H.fz, s));
     else if (vec)
       ODT_CUDA(launch_born_z_dyadic(a, dy, jj, H.fz, H.max_smem, s));
     else if (pipe_z && b16)
@@ -736,6 +739,8 @@ void run_chunk(Handle& H, int nb, cudaStream_t s, bool want_t, bool want_r, int 
     H.mark_begin(zkind, s);
     if (any_z)
       ODT_CUDA(launch_prime_z(a, jj, H.bsz.prime, s));
+    else if (pipe_zd)
+      ODT_CUDA(launch_z_dyadic(a, dy, jj, H.fz, s));
     else if (vec)
       ODT_CUDA(launch_born_z_dyadic(a, dy, jj, H.fz, H.max_smem, s));
     else if (pipe_z)
