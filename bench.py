@@ -35,16 +35,18 @@ GRID = [128, 128, 128]
 N_ILL = 49
 SEED = 0
 # algorithmic HBM bytes per voxel and launch of each Born kernel kind
-# (complex64 = 8 B): born_x reads T, Field_n, Field, V and writes T, Field_n,
-# Field; born_y / born_z read and write T once.  "_pipe" = the pipelined
-# (TMA-fed, persistent) variants of the same passes; "born_x_pipe_edge" = the
-# pipelined x-pass of iterations 2, 3 and the final pass (56 B nominal);
-# "born_xy" = the fused xy-pass (x-pass and both y-FFTs with the plane in
-# shared memory: the same 56 B as the x-pass), "born_xy_edge" its launches
-# for iterations 1-3 and the final pass.
-ALG_BYTES_PER_VOXEL = {"born_x": 56, "born_y": 16, "born_z": 16,
-                       "born_x_pipe": 56, "born_y_pipe": 16, "born_z_pipe": 16,
-                       "born_x_pipe_edge": 56, "born_xy": 56, "born_xy_edge": 56}
+# (complex64 = 8 B): born_x reads T, X, V and the incident field (the RI grid's
+# share of the padded grid) and writes T and X; born_y / born_z read and write
+# T once.  "_pipe" = the pipelined (TMA-fed, persistent) variants of the same
+# passes, "born_x_pipe_edge" the x-pass's final launch; "born_xy" = the fused
+# xy-pass (x-pass and both y-FFTs with the plane in shared memory: the same
+# bytes as the x-pass), "born_xy_edge" its first and final launches.
+ROI_SHARE = (128 / 152) ** 3
+XY_BYTES = 40 + 8 * ROI_SHARE
+ITER_BYTES = XY_BYTES + 16
+ALG_BYTES_PER_VOXEL = {"born_x": XY_BYTES, "born_y": 16, "born_z": 16,
+                       "born_x_pipe": XY_BYTES, "born_y_pipe": 16, "born_z_pipe": 16,
+                       "born_x_pipe_edge": XY_BYTES, "born_xy": XY_BYTES, "born_xy_edge": XY_BYTES}
 # the same with T and Field_n in 16-bit block floating point (4 B per value
 # plus one exponent byte per 8 values): xy-pass 4+4 (T) + 4+4 (Field_n) + 16
 # (Field) + 8 (V) + 0.5 (exponents) = 40.5 B, z-pass 8 + 0.25 = 8.25 B; one
@@ -270,7 +272,7 @@ def run_ours(args, rank, world, local_rank):
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic,
                      "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": dom_ms / dom_n,
-                     "iteration_frac": (72.0 * vox_step / (born_ms / 1e3) / 1e9) / peak},
+                     "iteration_frac": (ITER_BYTES * vox_step / (born_ms / 1e3) / 1e9) / peak},
         "kernel_ms_per_step": {k: v[0] for k, v in kt.items()},
         "gpu_launches": launches_per_step * args.steps,
         "clocks": clocks,
