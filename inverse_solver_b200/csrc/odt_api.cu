@@ -369,8 +369,8 @@ DevFft make_dev_fft(Handle& H, int n, int kind, const char* what) {
 
 // make_dev_fft for any length: a length with a prime factor above 31 gets a
 // plan in *bs and a DevFft with no passes, which no tile kernel accepts: the
-// direct products of prime_pass.cu where its tables fit shared memory (primes
-// up to about 280), else (and for ODT_KERNELS=generic) Bluestein's algorithm
+// direct products of prime_pass.cu where it applies (primes up to 251, lengths up
+// to about 510), else (and for ODT_KERNELS=generic) Bluestein's algorithm
 // (tables on the device, transforms of the 5-smooth length m >= 2 n - 1
 // through the line / column tiles).
 DevFft make_handle_fft(Handle& H, int n, int kind, const char* what, AnyFft* bs) {

@@ -1,5 +1,5 @@
-// Transforms along an axis whose length has one prime factor p above 31:
-// n = q p (q <= 13), as q-point butterflies and a direct p-point DFT that is a
+// Transforms along an axis whose length has one prime factor p from 37 to 251:
+// n = q p (q <= 13, tiles of up to 256 threads: n to about 510), as q-point butterflies and a direct p-point DFT that is a
 // small matrix product in shared memory (prime_pass.cu).
 #pragma once
 
@@ -20,7 +20,7 @@ struct PrimePlan {
 };
 
 // Host part of a plan (no device pointers); q == 0 where the kernel does not
-// apply (no such factorisation, or the tables and a tile of 16 pencils exceed
+// apply (no such factorisation, or a tile of 16 pencils exceeds the threads or
 // max_smem).
 PrimePlan prime_plan(int n, size_t max_smem);
 // Host tables of a plan: [2][h][kp] and a row of zeros.
