@@ -40,7 +40,7 @@ constexpr int kR1 = 8;                 // a tile of W x-lines takes W * 8 thread
                                        // one radix-R2 butterfly per thread
 
 struct PipeLine {      // per-line constants of a tile
-  long long g;         // element offset of x = 0 in T / Field_n / Field
+  long long g;         // element offset of x = 0 in T / X
   long long einc;      // Einc / Fout offset of x = 0 (when roi != 0)
   int v;               // element offset of x = 0 in V
   int valid;
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
   constexpr int kThreads = W * kR1;
   using L = PipeSmem<N, W>;
   extern __shared__ __align__(128) unsigned char sm[];
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::kBars);  // [0], [1]: T stages, [2]: Fn/F
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::kBars);  // [0], [1]: T stages, [2]: X
   float2* tw = reinterpret_cast<float2*>(sm + L::kTw);
   float2* r0t = reinterpret_cast<float2*>(sm + L::kR0);
   float* m0t = reinterpret_cast<float*>(sm + L::kM0);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(W * 8, W == 16 ? 2 : 3)
     // butterflies, slot s -> line 2 (s/16 / kJB) + (s%16)/8, butterfly
     // 8 (s/16 % kJB) + s%8.  The line pitch N = 8 (mod 16) elements puts the
     // other line 8 banks away, so every shared-memory access of the pass
-    // (T, Field_n, Field, the second buffer) hits 16 distinct 8-byte banks
+    // (T, X, the second buffer) hits 16 distinct 8-byte banks
     // per half-warp; slots with j >= R2 idle.  (kW / 2) kJB 16 slots take as
     // many rounds of kThreads as the kW R2 butterflies would.
     constexpr int kJB = (R2 + 7) / 8;

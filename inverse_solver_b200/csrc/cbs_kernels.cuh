@@ -119,10 +119,10 @@ cudaError_t launch_born_x(const BornArgs& a, int mode, int jj, const DevFft& fx,
 bool born_x_pipe_supported(const BornArgs& a, const DevFft& fx);
 cudaError_t launch_born_x_pipe(const BornArgs& a, int mode, int jj, const DevFft& fx, int* fault,
                                cudaStream_t s);
-// Pipelined column passes (persistent CTAs, tiled TMA copies) for lengths
-// 8 * {11, 15, 19, 25, 27} along y / z: the y-FFT of the Born loop in place on a.T,
-// and the z-pass; same results as launch_fft_cols / launch_born_z up to the
-// order of the radix passes of the inverse y-FFT.
+// Pipelined column passes (persistent CTAs, tiled TMA copies): the y-FFT of the
+// Born loop in place on a.T for lengths 8 * {11, 15, 19, 25, 27, 35}, and the z-pass
+// of the 16-bit storage (8 R, 11 <= R <= 20, 25, 27); same results as
+// launch_fft_cols / launch_born_z up to the order of the radix passes.
 bool cols_pipe_supported(const BornArgs& a, const DevFft& f, bool zpass);
 cudaError_t launch_fft_y_pipe(const BornArgs& a, bool inverse, const DevFft& fy, int* fault,
                               cudaStream_t s);
@@ -138,10 +138,10 @@ bool y_pass_supported(const BornArgs& a, const DevFft& f);
 cudaError_t launch_y_pass(const BornArgs& a, bool inverse, const DevFft& fy, int* fault, cudaStream_t s);
 // Fused xy-pass (born_xy.cu): the whole x-y plane of one z and illumination
 // in shared memory -- inverse y- and x-FFT of T, update of iteration jj-1,
-// source of iteration jj, forward x- and y-FFT -- for px == py = 8 * {11, 12,
-// 15, 19}; replaces launch_born_x and both y-FFTs (modes as launch_born_x;
-// the z-pass must run with a.perm_xy = 1).  Same results as the separate passes
-// up to the order of the FFT arithmetic.
+// source of iteration jj, forward x- and y-FFT -- for px == py = 8 R,
+// 5 <= R <= 28 (16-bit storage: 11 <= R <= 20); replaces launch_born_x and both
+// y-FFTs (modes as launch_born_x; the z-pass must run with a.perm_xy = 1).  Same
+// results as the separate passes up to the order of the FFT arithmetic.
 bool born_xy_supported(const BornArgs& a, int max_smem, bool b16);
 cudaError_t launch_born_xy(const BornArgs& a, int mode, int jj, const DevFft& fx, cudaStream_t s);
 // z-pass of iteration jj: forward z-FFT, Green's multiply, inverse z-FFT.
