@@ -22,11 +22,15 @@
 // m >= 2 p - 1 points and two chirps through shared memory) took 0.58 ms, and
 // the z-pass as two of those and a separate product 1.34 against 0.60 ms.
 //
-// The sums of at most 125 FP32 products are about as accurate as Bluestein's
-// transforms: relative error of random lines against double precision 0.9e-7
-// (p = 37), 1.3e-7 (89), 1.5e-7 (127), 1.8e-7 (181), 2.0e-7 (251), against 1.6e-7 to
-// 1.8e-7.  FP32 throughout; tcgen05 has no FP32 multiply, and its TF32 form
-// would need the operands in three parts.
+// Rounding of a sum of h FP32 products grows with p; Bluestein's hardly does.
+// Measured per axis on random data against double precision: 0.9e-7 (p = 37),
+// 1.3e-7 (89), 1.5e-7 (127) in one sum, but 1.6e-7 (151), 1.9e-7 (211), 2.1e-7
+// (251); Bluestein's transforms 1.8e-7 to 2.5e-7 on the device, 1.5e-7 to 1.8e-7
+// with ideal inner transforms.  Above p = 139 the sums therefore run in two
+// halves: 1.2e-7 (151), 1.4e-7 (211), 1.55e-7 (251), for 3 to 14 % of the axis's time
+// (20 M points, lines and columns: 151 points 0.280 -> 0.289 and 0.252 -> 0.287 ms, 251
+// points 0.365 -> 0.387 and 0.324 -> 0.351).  FP32 throughout; tcgen05 has no FP32
+// multiply, and its TF32 form would need the operands in three parts.
 #include <cmath>
 #include <type_traits>
 
@@ -41,9 +45,12 @@ namespace {
 constexpr int kKT = 8, kCT = 2;       // values of k, pencils per thread
 constexpr int kMaxThreads = 256;
 constexpr int kMaxQ = 13;
-// largest prime: beyond it the sums' rounding (2.0e-7 at 251) would pass the 1.6e-7
-// to 1.8e-7 of Bluestein's transforms by more than a fifth
+// largest prime whose rounding and speed were measured.  The work per value grows
+// with p, but has not met Bluestein's there: y axis of a 36 x n x 36 grid of 8
+// waves, Bluestein against direct, ms per launch: 0.063, 0.031 (n = 127), 0.079, 0.051
+// (151), 0.131, 0.062 (211), 0.130, 0.071 (251, in one sum; 0.077 in two halves)
 constexpr int kMaxP = 251;
+constexpr int kSplitP = 139;          // above it the sums run in two halves
 
 __host__ __device__ inline int pitch_of(int w, bool lines) { return lines ? w + 2 : w; }
 
@@ -63,7 +70,8 @@ struct AxisArgs {
 };
 
 // OP 0: one transform; 1: forward, Green's multiply, inverse (columns)
-template <bool LINES, int OP>
+// (HALVES: the sums over j in two parts, see kSplitP)
+template <bool LINES, int OP, bool HALVES>
 __global__ void __launch_bounds__(kMaxThreads, 2) prime_kernel(const AxisArgs g, const PrimePlan f, const BornArgs a,
                                                             const int jj) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -221,23 +229,54 @@ __global__ void __launch_bounds__(kMaxThreads, 2) prime_kernel(const AxisArgs g,
         pv -= pitch;
       };
       read();
+      auto sum = [&](int n) {
 #pragma unroll 2
-      for (int j = 1; j <= h; ++j) {
-        const float ck[kKT] = {cc[0].x, cc[0].y, cc[0].z, cc[0].w, cc[1].x, cc[1].y, cc[1].z, cc[1].w};
-        const float sk[kKT] = {ss[0].x, ss[0].y, ss[0].z, ss[0].w, ss[1].x, ss[1].y, ss[1].z, ss[1].w};
-        float2 u[kCT], v[kCT];
+        for (int j = 0; j < n; ++j) {
+          const float ck[kKT] = {cc[0].x, cc[0].y, cc[0].z, cc[0].w, cc[1].x, cc[1].y, cc[1].z, cc[1].w};
+          const float sk[kKT] = {ss[0].x, ss[0].y, ss[0].z, ss[0].w, ss[1].x, ss[1].y, ss[1].z, ss[1].w};
+          float2 u[kCT], v[kCT];
 #pragma unroll
-        for (int c = 0; c < kCT; ++c) {
-          u[c] = cadd(x[c], y[c]);
-          v[c] = csub(x[c], y[c]);
+          for (int c = 0; c < kCT; ++c) {
+            u[c] = cadd(x[c], y[c]);
+            v[c] = csub(x[c], y[c]);
+          }
+          read();
+#pragma unroll
+          for (int k = 0; k < kKT; ++k)
+#pragma unroll
+            for (int c = 0; c < kCT; ++c) {
+              C[k][c] = cfma_real(ck[k], u[c], C[k][c]);
+              S[k][c] = cfma_real(sk[k], v[c], S[k][c]);
+            }
         }
-        read();
+      };
+      if constexpr (!HALVES) {
+        sum(h);
+      } else {
+        // the first half's sums wait in local memory (64 stores and loads a
+        // thread; volatile, or the compiler keeps both halves in registers and
+        // spills inside the loop)
+        volatile float part[4 * kKT * kCT];
+        sum(h / 2);
 #pragma unroll
         for (int k = 0; k < kKT; ++k)
 #pragma unroll
           for (int c = 0; c < kCT; ++c) {
-            C[k][c] = cfma_real(ck[k], u[c], C[k][c]);
-            S[k][c] = cfma_real(sk[k], v[c], S[k][c]);
+            const int i = 4 * (k * kCT + c);
+            part[i] = C[k][c].x;
+            part[i + 1] = C[k][c].y;
+            part[i + 2] = S[k][c].x;
+            part[i + 3] = S[k][c].y;
+            C[k][c] = S[k][c] = make_float2(0.f, 0.f);
+          }
+        sum(h - h / 2);
+#pragma unroll
+        for (int k = 0; k < kKT; ++k)
+#pragma unroll
+          for (int c = 0; c < kCT; ++c) {
+            const int i = 4 * (k * kCT + c);
+            C[k][c] = make_float2(C[k][c].x + part[i], C[k][c].y + part[i + 1]);
+            S[k][c] = make_float2(S[k][c].x + part[i + 2], S[k][c].y + part[i + 3]);
           }
       }
     };
@@ -334,22 +373,27 @@ __global__ void __launch_bounds__(kMaxThreads, 2) prime_kernel(const AxisArgs g,
   }
 }
 
-template <bool LINES, int OP>
-cudaError_t launch(const AxisArgs& g, const PrimePlan& f, const BornArgs& a, int jj, cudaStream_t s) {
+template <bool LINES, int OP, bool HALVES>
+cudaError_t launch_sums(const AxisArgs& g, const PrimePlan& f, const BornArgs& a, int jj, cudaStream_t s) {
   const size_t sm = smem_of(f, f.w);
   const int unit = f.w > 32 ? f.w : 32;
   const int nthr = (items_of(f, f.w) + unit - 1) / unit * unit;
-  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(prime_kernel<LINES, OP>), sm);
+  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(prime_kernel<LINES, OP, HALVES>), sm);
   if (e != cudaSuccess) return e;
   int dev = 0, nsm = 0, per_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prime_kernel<LINES, OP>, nthr, sm);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prime_kernel<LINES, OP, HALVES>, nthr, sm);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const long long cap = (long long)per_sm * nsm;
-  prime_kernel<LINES, OP><<<(unsigned)(g.ntiles < cap ? g.ntiles : cap), nthr, sm, s>>>(g, f, a, jj);
+  prime_kernel<LINES, OP, HALVES><<<(unsigned)(g.ntiles < cap ? g.ntiles : cap), nthr, sm, s>>>(g, f, a, jj);
   return cudaGetLastError();
+}
+
+template <bool LINES, int OP>
+cudaError_t launch(const AxisArgs& g, const PrimePlan& f, const BornArgs& a, int jj, cudaStream_t s) {
+  return f.p > kSplitP ? launch_sums<LINES, OP, true>(g, f, a, jj, s) : launch_sums<LINES, OP, false>(g, f, a, jj, s);
 }
 
 }  // namespace
