@@ -15,7 +15,7 @@
 // bounds the accuracy of the transform; nothing here calls sin/cos).
 //
 // Radices: 2, 4, 8 (closed-form butterflies), composite ones from two smaller
-// butterflies, and odd primes <= 31 through the
+// butterflies, and 9 and odd primes <= 31 through the
 // symmetric real-coefficient DFT (pairs v[m], v[R-m] so that an odd R-point
 // DFT costs (R-1)^2 real multiply-adds instead of R^2 complex products).
 //
@@ -239,7 +239,7 @@ struct Butterfly<12, INV> {
   }
 };
 
-// Odd prime R: X[k] = v0 + sum_m a_m cos(2 pi m k / R) -/+ i sum_m b_m sin(2 pi m k / R)
+// Odd R (primes and 9): X[k] = v0 + sum_m a_m cos(2 pi m k / R) -/+ i sum_m b_m sin(2 pi m k / R)
 // with a_m = v[m] + v[R-m], b_m = v[m] - v[R-m]; the cosines and sines are
 // read from the transform's table at multiples of n / R.
 template <int R, bool INV>
@@ -250,7 +250,7 @@ struct OddButterfly {
     (void)tw;
     (void)n;
     float cs[H + 1], sn[H + 1];
-    cs[0] = 1.f;
+    cs[0] = 1.f;  // m*k can be a multiple of R when R is composite
     sn[0] = 0.f;
 #pragma unroll
     for (int t = 1; t <= H; ++t) {
@@ -292,25 +292,76 @@ struct OddButterfly {
   }
 };
 
-// A * B points in registers (Cooley-Tukey with both factors as butterflies):
-// n = B n1 + n2, k = k1 + A k2; A-point DFTs over n1, the twiddles
-// W_AB^(n2 k1) as compile-time constants, B-point DFTs over n2.  For
-// composite radices of the pipelined passes (35 = 5 x 7: the 280-point axes).
+// The butterflies inside a composite one: 3 and 5 points with sin(pi / 3) and
+// sin(2 pi / 5) split in two, because the one that is rounded to float is short by
+// 1.8e-8 (long by 2.5e-8) in every product, and nested or repeated transforms
+// add that up (27 = 3 x 9 forth and back: gain -4.2e-8, with the split -1.0e-8).
+template <int R, bool INV>
+struct InnerButterfly : Butterfly<R, INV> {};
+
+template <bool INV>
+struct InnerButterfly<3, INV> {
+  ODT_HD static void run(float2* v, const float2*, int) {
+    const float lo = (float)(0.875 - 0.86602540378443864676);
+    const float2 x0 = v[0], a = cadd(v[1], v[2]);
+    // j = -/+ i (v1 - v2)
+    const float2 j = INV ? make_float2(v[2].y - v[1].y, v[1].x - v[2].x) : make_float2(v[1].y - v[2].y, v[2].x - v[1].x);
+    const float2 m = cfma_real(-0.5f, a, x0);
+    v[0] = cadd(x0, a);
+    v[1] = cfma_real(-lo, j, cfma_real(0.875f, j, m));
+    v[2] = cfma_real(lo, j, cfma_real(-0.875f, j, m));
+  }
+};
+
+template <bool INV>
+struct InnerButterfly<5, INV> {
+  ODT_HD static void run(float2* v, const float2*, int) {
+    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
+    const float s2 = 0.58778525229247312917f, lo = (float)(1 - 0.95105651629515357212);
+    const float2 x0 = v[0], a1 = cadd(v[1], v[4]), a2 = cadd(v[2], v[3]);
+    const float2 j1 = INV ? make_float2(v[4].y - v[1].y, v[1].x - v[4].x) : make_float2(v[1].y - v[4].y, v[4].x - v[1].x);
+    const float2 j2 = INV ? make_float2(v[3].y - v[2].y, v[2].x - v[3].x) : make_float2(v[2].y - v[3].y, v[3].x - v[2].x);
+    const float2 p1 = cfma_real(c2, a2, cfma_real(c1, a1, x0)), p2 = cfma_real(c1, a2, cfma_real(c2, a1, x0));
+    const float2 q1 = cfma_real(-lo, j1, cfma_real(s2, j2, j1));               // sin(2 pi / 5) j1 + s2 j2
+    const float2 q2 = cfma_real(lo, j2, csub(cscale(j1, s2), j2));             // s2 j1 - sin(2 pi / 5) j2
+    v[0] = cadd(cadd(x0, a1), a2);
+    v[1] = cadd(p1, q1);
+    v[4] = csub(p1, q1);
+    v[2] = cadd(p2, q2);
+    v[3] = csub(p2, q2);
+  }
+};
+
+constexpr int ce_gcd(int a, int b) { return b == 0 ? a : ce_gcd(b, a % b); }
+constexpr int ce_inverse(int a, int m) {   // a^-1 mod m
+  for (int i = 1; i < m; ++i)
+    if (a * i % m == 1) return i;
+  return 0;
+}
+
+// A * B points in registers, both factors as butterflies.  Coprime factors: the
+// prime-factor algorithm (Good 1958), n = B n1 + A n2 and k = k1 B (B^-1 mod A) +
+// k2 A (A^-1 mod B) mod AB, which has no twiddles.  Else Cooley-Tukey: n = B n1 + n2,
+// k = k1 + A k2, the twiddles W_AB^(n2 k1) as compile-time constants.  Every
+// inner twiddle is another rounding: 20 points forth and back 1.04e-7 with
+// twiddles, 0.89e-7 without.
 template <int A, int B, bool INV>
 struct CompositeButterfly {
   ODT_HD static void run(float2* v, const float2* tw, int n) {
     constexpr int AB = A * B;
+    constexpr bool kCoprime = ce_gcd(A, B) == 1;
+    constexpr int kA = B * ce_inverse(B % A, A), kB = A * ce_inverse(A % B, B);
     constexpr UnitRoots<AB> ur{};
     float2 t[B][A];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) {
       float2 q[A];
 #pragma unroll
-      for (int n1 = 0; n1 < A; ++n1) q[n1] = v[B * n1 + n2];
-      Butterfly<A, INV>::run(q, tw, n);
+      for (int n1 = 0; n1 < A; ++n1) q[n1] = v[kCoprime ? (B * n1 + A * n2) % AB : B * n1 + n2];
+      InnerButterfly<A, INV>::run(q, tw, n);
 #pragma unroll
       for (int k1 = 0; k1 < A; ++k1) {
-        const int e = (n2 * k1) % AB;
+        const int e = kCoprime ? 0 : (n2 * k1) % AB;
         if (e == 0) {
           t[n2][k1] = q[k1];
         } else {   // exp(-/+ 2 pi i e / AB)
@@ -324,9 +375,9 @@ struct CompositeButterfly {
       float2 q[B];
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2) q[n2] = t[n2][k1];
-      Butterfly<B, INV>::run(q, tw, n);
+      InnerButterfly<B, INV>::run(q, tw, n);
 #pragma unroll
-      for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = q[k2];
+      for (int k2 = 0; k2 < B; ++k2) v[kCoprime ? (k1 * kA + k2 * kB) % AB : k1 + A * k2] = q[k2];
     }
   }
 };
@@ -341,6 +392,7 @@ struct CompositeButterfly {
 ODT_ODD_BUTTERFLY(3)
 ODT_ODD_BUTTERFLY(5)
 ODT_ODD_BUTTERFLY(7)
+ODT_ODD_BUTTERFLY(9)
 ODT_ODD_BUTTERFLY(11)
 ODT_ODD_BUTTERFLY(13)
 ODT_ODD_BUTTERFLY(17)
@@ -351,16 +403,19 @@ ODT_ODD_BUTTERFLY(31)
 #undef ODT_ODD_BUTTERFLY
 
 // Composite radices.  The symmetric DFT costs (R - 1)^2 real multiply-adds,
-// the two-factor form A (B - 1)^2 + B (A - 1)^2 and four operations per inner
-// twiddle: 676 against about 300 for 27 = 3 x 9, 576 against 224 for 25,
-// 196 against 100 for 15, 64 against 40 for 9.
+// the two-factor form A (B - 1)^2 + B (A - 1)^2 and, where the factors have a
+// common divisor, four operations per inner twiddle: 676 against about 300 for
+// 27 = 3 x 9, 576 against 224 for 25, 196 against 78 for 15.  Forth and back on
+// random data they round like the symmetric form: 1.11e-7 against 1.12e-7 (27),
+// 1.08e-7 against 1.08e-7 (25), 0.94e-7 against 0.92e-7 (15).  9 points stay
+// symmetric: 3 x 3 saves 24 of 64 multiply-adds but rounds worse (0.99e-7
+// against 0.80e-7).
 #define ODT_COMPOSITE_BUTTERFLY(A, B)                                                                      \
   template <bool INV>                                                                                     \
   struct Butterfly<A * B, INV> {                                                                          \
     ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<A, B, INV>::run(v, tw, n); } \
   };
 ODT_COMPOSITE_BUTTERFLY(2, 3)
-ODT_COMPOSITE_BUTTERFLY(3, 3)
 ODT_COMPOSITE_BUTTERFLY(2, 5)
 ODT_COMPOSITE_BUTTERFLY(2, 7)
 ODT_COMPOSITE_BUTTERFLY(3, 5)
