@@ -198,47 +198,6 @@ struct UnitRoots {   // cos / sin of 2 pi t / R, t < R, as float
   }
 };
 
-// R = 12 = 4 x 3 in registers (for the fused passes on lengths 96 = 8 x 12):
-// n = 3 n1 + n2, k = k1 + 4 k2; 4-point DFTs over n1, twiddles W_12^(n2 k1)
-// as compile-time constants, 3-point DFTs over n2.
-template <bool INV>
-struct Butterfly<12, INV> {
-  ODT_HD static void run(float2* v, const float2* tw, int n) {
-    constexpr UnitRoots<12> ur{};
-    (void)tw;
-    (void)n;
-    float2 t[3][4];
-#pragma unroll
-    for (int n2 = 0; n2 < 3; ++n2) {
-      float2 q[4] = {v[n2], v[3 + n2], v[6 + n2], v[9 + n2]};
-      Butterfly<4, INV>::run(q, nullptr, 0);
-#pragma unroll
-      for (int k1 = 0; k1 < 4; ++k1) {
-        const int e = n2 * k1;
-        if (e == 0) {
-          t[n2][k1] = q[k1];
-        } else {   // exp(-/+ 2 pi i e / 12)
-          const float2 w = make_float2(ur.c[e], INV ? ur.s[e] : -ur.s[e]);
-          t[n2][k1] = cmul(q[k1], w);
-        }
-      }
-    }
-    // 3-point DFT: c = cos(2 pi / 3) = -1/2, s = sin(2 pi / 3)
-    const float s3 = 0.86602540378443864676f;
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) {
-      const float2 a0 = t[0][k1], a1 = t[1][k1], a2 = t[2][k1];
-      const float2 sum = cadd(a1, a2), dif = csub(a1, a2);
-      const float2 m = make_float2(a0.x - 0.5f * sum.x, a0.y - 0.5f * sum.y);
-      // forward: X1 = m - i s dif, X2 = m + i s dif
-      const float2 j = make_float2(-s3 * dif.y, s3 * dif.x);   // i s dif
-      v[k1] = cadd(a0, sum);
-      v[k1 + 4] = INV ? cadd(m, j) : csub(m, j);
-      v[k1 + 8] = INV ? csub(m, j) : cadd(m, j);
-    }
-  }
-};
-
 // Odd R (primes and 9): X[k] = v0 + sum_m a_m cos(2 pi m k / R) -/+ i sum_m b_m sin(2 pi m k / R)
 // with a_m = v[m] + v[R-m], b_m = v[m] - v[R-m]; the cosines and sines are
 // read from the transform's table at multiples of n / R.
@@ -292,15 +251,19 @@ struct OddButterfly {
   }
 };
 
-// The butterflies inside a composite one: 3 and 5 points with sin(pi / 3) and
-// sin(2 pi / 5) split in two, because the one that is rounded to float is short by
-// 1.8e-8 (long by 2.5e-8) in every product, and nested or repeated transforms
-// add that up (27 = 3 x 9 forth and back: gain -4.2e-8, with the split -1.0e-8).
+// Butterflies of 3, 5 and 8 points whose irrational constant is held in two parts.
+// Rounded to float, sin(pi / 3) is short by 1.8e-8, sin(2 pi / 5) long by 2.5e-8 and
+// sqrt(1 / 2) short by 1.7e-8, in every product, and transforms that are nested
+// or repeated add that up (27 = 3 x 9 forth and back: gain -4.2e-8, so -1.0e-8).
+// They serve as factors of composite butterflies and in beam propagation,
+// whose slices transform the same field back and forth.  The second
+// multiply-add is another rounding (8 points forth and back 0.64e-7, so
+// 0.68e-7), so all other steps keep the plain ones.
 template <int R, bool INV>
-struct InnerButterfly : Butterfly<R, INV> {};
+struct FineButterfly : Butterfly<R, INV> {};
 
 template <bool INV>
-struct InnerButterfly<3, INV> {
+struct FineButterfly<3, INV> {
   ODT_HD static void run(float2* v, const float2*, int) {
     const float lo = (float)(0.875 - 0.86602540378443864676);
     const float2 x0 = v[0], a = cadd(v[1], v[2]);
@@ -314,7 +277,7 @@ struct InnerButterfly<3, INV> {
 };
 
 template <bool INV>
-struct InnerButterfly<5, INV> {
+struct FineButterfly<5, INV> {
   ODT_HD static void run(float2* v, const float2*, int) {
     const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
     const float s2 = 0.58778525229247312917f, lo = (float)(1 - 0.95105651629515357212);
@@ -332,36 +295,63 @@ struct InnerButterfly<5, INV> {
   }
 };
 
+template <bool INV>
+struct FineButterfly<8, INV> {
+  ODT_HD static void run(float2* v, const float2*, int) {
+    const float lo = (float)(0.70710678118654752440 - 0.6875);
+    float2 e[4] = {v[0], v[2], v[4], v[6]};
+    float2 o[4] = {v[1], v[3], v[5], v[7]};
+    Butterfly<4, INV>::run(e, nullptr, 0);
+    Butterfly<4, INV>::run(o, nullptr, 0);
+    // as Butterfly<8>: o1 and o3 hold W8^k o[k] sqrt(2)
+    const float2 o1 = INV ? make_float2(o[1].x - o[1].y, o[1].x + o[1].y) : make_float2(o[1].x + o[1].y, o[1].y - o[1].x);
+    const float2 o3 =
+        INV ? make_float2(-(o[3].x + o[3].y), o[3].x - o[3].y) : make_float2(o[3].y - o[3].x, -(o[3].x + o[3].y));
+    v[0] = cadd(e[0], o[0]);
+    v[4] = csub(e[0], o[0]);
+    v[1] = cfma_real(lo, o1, cfma_real(0.6875f, o1, e[1]));
+    v[5] = cfma_real(-lo, o1, cfma_real(-0.6875f, o1, e[1]));
+    v[2] = addrot<INV>(e[2], o[2]);
+    v[6] = subrot<INV>(e[2], o[2]);
+    v[3] = cfma_real(lo, o3, cfma_real(0.6875f, o3, e[3]));
+    v[7] = cfma_real(-lo, o3, cfma_real(-0.6875f, o3, e[3]));
+  }
+};
+
 constexpr int ce_gcd(int a, int b) { return b == 0 ? a : ce_gcd(b, a % b); }
 constexpr int ce_inverse(int a, int m) {   // a^-1 mod m
   for (int i = 1; i < m; ++i)
     if (a * i % m == 1) return i;
   return 0;
 }
+template <int A, int B>
+struct PrimeFactorMap {   // output index (k1 kA + k2 kB) mod AB of the prime-factor algorithm
+  static constexpr bool kCoprime = ce_gcd(A, B) == 1;
+  static constexpr int kA = B * ce_inverse(B % A, A), kB = A * ce_inverse(A % B, B);
+};
 
 // A * B points in registers, both factors as butterflies.  Coprime factors: the
 // prime-factor algorithm (Good 1958), n = B n1 + A n2 and k = k1 B (B^-1 mod A) +
 // k2 A (A^-1 mod B) mod AB, which has no twiddles.  Else Cooley-Tukey: n = B n1 + n2,
 // k = k1 + A k2, the twiddles W_AB^(n2 k1) as compile-time constants.  Every
 // inner twiddle is another rounding: 20 points forth and back 1.04e-7 with
-// twiddles, 0.89e-7 without.
-template <int A, int B, bool INV>
+// twiddles, 0.90e-7 without.
+template <int A, int B, bool INV, template <int, bool> class F = FineButterfly>
 struct CompositeButterfly {
   ODT_HD static void run(float2* v, const float2* tw, int n) {
     constexpr int AB = A * B;
-    constexpr bool kCoprime = ce_gcd(A, B) == 1;
-    constexpr int kA = B * ce_inverse(B % A, A), kB = A * ce_inverse(A % B, B);
+    using M = PrimeFactorMap<A, B>;
     constexpr UnitRoots<AB> ur{};
     float2 t[B][A];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) {
       float2 q[A];
 #pragma unroll
-      for (int n1 = 0; n1 < A; ++n1) q[n1] = v[kCoprime ? (B * n1 + A * n2) % AB : B * n1 + n2];
-      InnerButterfly<A, INV>::run(q, tw, n);
+      for (int n1 = 0; n1 < A; ++n1) q[n1] = v[M::kCoprime ? (B * n1 + A * n2) % AB : B * n1 + n2];
+      F<A, INV>::run(q, tw, n);
 #pragma unroll
       for (int k1 = 0; k1 < A; ++k1) {
-        const int e = kCoprime ? 0 : (n2 * k1) % AB;
+        const int e = M::kCoprime ? 0 : (n2 * k1) % AB;
         if (e == 0) {
           t[n2][k1] = q[k1];
         } else {   // exp(-/+ 2 pi i e / AB)
@@ -375,9 +365,9 @@ struct CompositeButterfly {
       float2 q[B];
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2) q[n2] = t[n2][k1];
-      InnerButterfly<B, INV>::run(q, tw, n);
+      F<B, INV>::run(q, tw, n);
 #pragma unroll
-      for (int k2 = 0; k2 < B; ++k2) v[kCoprime ? (k1 * kA + k2 * kB) % AB : k1 + A * k2] = q[k2];
+      for (int k2 = 0; k2 < B; ++k2) v[M::kCoprime ? (k1 * M::kA + k2 * M::kB) % AB : k1 + A * k2] = q[k2];
     }
   }
 };
@@ -410,18 +400,24 @@ ODT_ODD_BUTTERFLY(31)
 // 1.08e-7 against 1.08e-7 (25), 0.94e-7 against 0.92e-7 (15).  9 points stay
 // symmetric: 3 x 3 saves 24 of 64 multiply-adds but rounds worse (0.99e-7
 // against 0.80e-7).
-#define ODT_COMPOSITE_BUTTERFLY(A, B)                                                                      \
+#define ODT_COMPOSITE_BUTTERFLY_OF(A, B, F)                                                                      \
   template <bool INV>                                                                                     \
   struct Butterfly<A * B, INV> {                                                                          \
-    ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<A, B, INV>::run(v, tw, n); } \
+    ODT_HD static void run(float2* v, const float2* tw, int n) { CompositeButterfly<A, B, INV, F>::run(v, tw, n); } \
   };
+// 10, 20, 30 and 35 points keep the plain 5-point factor: its long sine makes up
+// for the short constants of the 8-point step beside it (Born series on padded
+// 160 x 160 x 96, rounding against double precision: 0.80e-7, with the split
+// one 0.96e-7).
+#define ODT_COMPOSITE_BUTTERFLY(A, B) ODT_COMPOSITE_BUTTERFLY_OF(A, B, FineButterfly)
 ODT_COMPOSITE_BUTTERFLY(2, 3)
-ODT_COMPOSITE_BUTTERFLY(2, 5)
+ODT_COMPOSITE_BUTTERFLY_OF(2, 5, Butterfly)
+ODT_COMPOSITE_BUTTERFLY(4, 3)
 ODT_COMPOSITE_BUTTERFLY(2, 7)
 ODT_COMPOSITE_BUTTERFLY(3, 5)
 ODT_COMPOSITE_BUTTERFLY(4, 4)
 ODT_COMPOSITE_BUTTERFLY(2, 9)
-ODT_COMPOSITE_BUTTERFLY(4, 5)
+ODT_COMPOSITE_BUTTERFLY_OF(4, 5, Butterfly)
 ODT_COMPOSITE_BUTTERFLY(3, 7)
 ODT_COMPOSITE_BUTTERFLY(2, 11)
 ODT_COMPOSITE_BUTTERFLY(3, 8)
@@ -429,8 +425,8 @@ ODT_COMPOSITE_BUTTERFLY(5, 5)
 ODT_COMPOSITE_BUTTERFLY(2, 13)
 ODT_COMPOSITE_BUTTERFLY(3, 9)
 ODT_COMPOSITE_BUTTERFLY(4, 7)
-ODT_COMPOSITE_BUTTERFLY(5, 6)
-ODT_COMPOSITE_BUTTERFLY(5, 7)
+ODT_COMPOSITE_BUTTERFLY_OF(5, 6, Butterfly)
+ODT_COMPOSITE_BUTTERFLY_OF(5, 7, Butterfly)
 #undef ODT_COMPOSITE_BUTTERFLY
 
 // ------------------------------------------------------------------ one pass
