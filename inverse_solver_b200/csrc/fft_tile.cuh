@@ -141,7 +141,8 @@ struct Thr {
   int tid, nthr;
 };
 
-template <int R, bool INV, class Map, class Src, class Dst>
+// (BF: the family of butterflies, see FineButterfly)
+template <int R, bool INV, template <int, bool> class BF = Butterfly, class Map, class Src, class Dst>
 ODT_HD void tile_pass(const Thr& th, const Map& m, int n, int ns, const float2* tw,
                       const Src& src, const Dst& dst) {
   const int nb = n / R;
@@ -168,7 +169,7 @@ ODT_HD void tile_pass(const Thr& th, const Map& m, int n, int ns, const float2* 
         v[r] = cmul(v[r], w);
       }
     }
-    Butterfly<R, INV>::run(v, tw, n);
+    BF<R, INV>::run(v, tw, n);
     const int d = (j - k) * R + k;
 #pragma unroll
     for (int r = 0; r < R; ++r) dst.store(d + r * ns, c, v[r]);
@@ -184,7 +185,8 @@ ODT_HD void tile_pass(const Thr& th, const Map& m, int n, int ns, const float2* 
 //            (forward) pass; MODE_END: last pass -> op, nothing stored.
 enum MidMode { kMidBoth = 0, kMidGen = 1, kMidEnd = 2 };
 
-template <int R, bool FIRST_INV, int MODE, class Map, class Src, class Dst, class Op>
+template <int R, bool FIRST_INV, int MODE, template <int, bool> class BF = Butterfly, class Map, class Src, class Dst,
+          class Op>
 ODT_HD void tile_mid(const Thr& th, const Map& m, int n, const float2* tw, const Src& src,
                      const Dst& dst, const Op& op) {
   const int nb = n / R;
@@ -211,14 +213,14 @@ ODT_HD void tile_mid(const Thr& th, const Map& m, int n, const float2* tw, const
           v[r] = cmul(v[r], w);
         }
       }
-      Butterfly<R, FIRST_INV>::run(v, tw, n);
+      BF<R, FIRST_INV>::run(v, tw, n);
     }
     op.template apply<R>(c, j, nb, v);
     if (MODE != kMidEnd) {
       if (MODE == kMidGen)
-        Butterfly<R, false>::run(v, tw, n);
+        BF<R, false>::run(v, tw, n);
       else
-        Butterfly<R, !FIRST_INV>::run(v, tw, n);
+        BF<R, !FIRST_INV>::run(v, tw, n);
 #pragma unroll
       for (int r = 0; r < R; ++r) dst.store(j * R + r, c, v[r]);
     }
@@ -272,16 +274,17 @@ ODT_HD void tile_mid(const Thr& th, const Map& m, int n, const float2* tw, const
       break;                                                                       \
   }
 
-template <int CLS, bool INV, class Map, class Src, class Dst>
+template <int CLS, bool INV, template <int, bool> class BF = Butterfly, class Map, class Src, class Dst>
 ODT_HD void tile_pass_any(const Thr& th, int R, const Map& m, int n, int ns, const float2* tw,
                           const Src& src, const Dst& dst) {
-  ODT_RADIX_SWITCH(R, CLS, (tile_pass<RR, INV>(th, m, n, ns, tw, src, dst)))
+  ODT_RADIX_SWITCH(R, CLS, (tile_pass<RR, INV, BF>(th, m, n, ns, tw, src, dst)))
 }
 
-template <int CLS, bool FIRST_INV, int MODE, class Map, class Src, class Dst, class Op>
+template <int CLS, bool FIRST_INV, int MODE, template <int, bool> class BF = Butterfly, class Map, class Src, class Dst,
+          class Op>
 ODT_HD void tile_mid_any(const Thr& th, int R, const Map& m, int n, const float2* tw,
                          const Src& src, const Dst& dst, const Op& op) {
-  ODT_RADIX_SWITCH(R, CLS, (tile_mid<RR, FIRST_INV, MODE>(th, m, n, tw, src, dst, op)))
+  ODT_RADIX_SWITCH(R, CLS, (tile_mid<RR, FIRST_INV, MODE, BF>(th, m, n, tw, src, dst, op)))
 }
 
 }  // namespace odt
