@@ -79,13 +79,6 @@ __device__ __forceinline__ void tma_tile(void* dst, const CUtensorMap* map, int 
 __device__ __forceinline__ void copy8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
-// Reciprocal: the hardware approximation (at most 1 ulp) and one Newton step.
-// The argument is q^2 + eps^2 >= eps^2, far from zero, subnormals, infinity.
-__device__ __forceinline__ float recip(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.f), r);
-}
 #endif
 
 inline PFN_cuTensorMapEncodeTiled_v12000 encoder() {

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R>())
           for (int r = 0; r < R; ++r) {
             float q = qxy + kz[k1 + A * r];
             q = a.g_scale * q - a.g_off;
-            const float rden = recip(q * q + a.eps * a.eps) * a.inv_n;
+            const float rden = __frcp_rn(q * q + a.eps * a.eps) * a.inv_n;
             v[r] = cmul(make_float2(q * rden, a.eps * rden), v[r]);  // (1 / (q - i eps)) / N
           }
           Butterfly<R, true>::run(v, tw, kN);
