@@ -684,8 +684,8 @@ odt_status odt_set_field_storage(odt_handle h, int32_t storage);
  * the separate pipelined x-, y-, z-passes, the generic tile kernels -- on
  * the potential set last, keeps the fastest for the handle's later solves
  * and caches the choice process-wide per (device, padded grid, batch,
- * components, storage), so a later handle of the same shape takes it without
- * timing.  The plans give the same results up to the order of the FFT
+ * components, storage, RI tensor or not), so a later handle of the same shape
+ * takes it without timing.  The plans give the same results up to the order of the FFT
  * arithmetic.  ms[i] is the time per solve of plan i (0: fused xy-pass, 1:
  * separate pipelined passes, 2: generic tile kernels; -1 where a plan does
  * not apply or was not timed).  Needs odt_set_potential first; synchronous. */

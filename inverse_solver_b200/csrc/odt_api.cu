@@ -1535,11 +1535,13 @@ odt_status odt_get_batch(odt_handle h, int32_t* batch) {
 }
 
 namespace {
-// process-wide plan choices of odt_autotune
+// process-wide plan choices of odt_autotune (an RI tensor has no fused
+// xy-pass, so its choice is not a scalar potential's)
 struct TuneKey {
-  int dev, px, py, pz, nb, np, storage;
+  int dev, px, py, pz, nb, np, storage, tensor;
   bool operator<(const TuneKey& o) const {
-    return std::tie(dev, px, py, pz, nb, np, storage) < std::tie(o.dev, o.px, o.py, o.pz, o.nb, o.np, o.storage);
+    return std::tie(dev, px, py, pz, nb, np, storage, tensor) <
+           std::tie(o.dev, o.px, o.py, o.pz, o.nb, o.np, o.storage, o.tensor);
   }
 };
 std::mutex g_tune_mu;
@@ -1556,7 +1558,8 @@ odt_status odt_autotune(odt_handle h, int32_t n_ill, odt_tune_result* out) {
     DeviceGuard dg(H->g.device);
     const int nb = std::min<int>(n_ill, auto_batch(*H, n_ill));
     ensure_batch(*H, nb);
-    const TuneKey key{H->g.device, H->g.sim_size[0], H->g.sim_size[1], H->g.sim_size[2], nb, H->np, H->storage};
+    const TuneKey key{H->g.device, H->g.sim_size[0], H->g.sim_size[1], H->g.sim_size[2], nb, H->np, H->storage,
+                      H->pot[0].tensor ? 1 : 0};
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       auto it = g_tune.find(key);
