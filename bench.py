@@ -55,6 +55,13 @@ ALG_BYTES_B16 = {"born_xy": 40.5, "born_xy_edge": 40.5, "born_z_pipe": 8.25}
 ITER_BYTES_B16 = 48.75
 
 
+def propagations(bornmax):
+    """Propagations that a complex64 solve of `bornmax` iterations runs: the
+    nested series starts with iteration 2, one of up to two iterations with
+    the first.  (16-bit storage goes term by term and runs every iteration.)"""
+    return bornmax - 1 if bornmax >= 3 else bornmax
+
+
 def workload_params():
     from inverse_solver_b200.forward import CBSHostSetup
 
@@ -264,7 +271,7 @@ def run_ours(args, rank, world, local_rank):
         "config": {"workload": workload_name(), "grid": GRID, "padded_grid": s.sim_size,
                    "n_ill": n_ill, "bornmax": s.Bornmax, "voxel_iters_per_step": vox_step,
                    "batch": s.batch(), "l2": "inputs larger than L2 (per-step working set "
-                   f"{3 * 8 * int(np.prod(s.sim_size)) * s.batch() / 1e9:.1f} GB)",
+                   f"{2 * 8 * int(np.prod(s.sim_size)) * s.batch() / 1e9:.1f} GB)",
                    "parallelism": f"dp{world} (illuminations, replicas)"},
         "latency_ms": {"p50": float(np.percentile(step_ms, 50)),
                        "p99": float(np.percentile(step_ms, 99))},
@@ -272,7 +279,8 @@ def run_ours(args, rank, world, local_rank):
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic,
                      "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": dom_ms / dom_n,
-                     "iteration_frac": (ITER_BYTES * vox_step / (born_ms / 1e3) / 1e9) / peak},
+                     "iteration_frac": (ITER_BYTES * vox_step * propagations(s.Bornmax) / max(1, s.Bornmax)
+                                        / (born_ms / 1e3) / 1e9) / peak},
         "kernel_ms_per_step": {k: v[0] for k, v in kt.items()},
         "gpu_launches": launches_per_step * args.steps,
         "clocks": clocks,
@@ -472,7 +480,7 @@ def run_bpm(args):
 
 GRID_LENGTH_CASES = (
     (72, "96^3 padded: fused xy-pass (12-point butterflies) + pipelined z-pass"),
-    (103, "127^3 padded: 127 is prime, Bluestein transforms on every axis, unfused Born loop"),
+    (103, "127^3 padded: 127 is prime, direct products on every axis"),
     (104, "128^3 padded: fused xy-pass + pipelined z-pass (16-point butterflies)"),
     (112, "136^3 padded: fused xy-pass + pipelined z-pass (17-point butterflies)"),
     (128, "152^3 padded: fused xy-pass + pipelined z-pass"),
@@ -485,14 +493,13 @@ def run_grid_lengths(args):
     of 16 ring illuminations (NA 1.2, 0.1 um voxels, seeded multi-sphere
     phantom, default boundary) on RI grids of 72^3, 103^3, 104^3, 112^3,
     128^3 and 136^3, which the default boundary pads to 96^3, 127^3 (prime:
-    Bluestein transforms), 128^3, 136^3, 152^3 and 160^3 (fused passes on all
+    direct products), 128^3, 136^3, 152^3 and 160^3 (fused passes on all
     but 127^3).  Device-resident solve_device calls
     timed with CUDA events;
     each solve moves more than the L2 (16 fields of >= 127^3 complex64).
     "kinds_one_solve" is one further solve with events around each kind of
-    launch; on the 127^3 grid the unfused loop books born_point under
-    born_x, each 3D FFT (three axis transforms) under born_y and born_green
-    under born_z."""
+    launch; on the 127^3 grid born_x holds the x transforms both ways and the
+    pointwise pass between them, born_y the y transforms, born_z the z-pass."""
     import torch
 
     from inverse_solver_b200 import FORWARD_SOLVER_CONVERGENT_BORN
