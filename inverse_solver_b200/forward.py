@@ -262,7 +262,7 @@ class CBSHostSetup:
         old = list(self.expected_RI_size)
         self.ROI = [btp[0] + 1, btp[0] + old[0], btp[1] + 1, btp[1] + old[1], btp[2] + 1, btp[2] + old[2]]
         shape, ub, masks, ramps, kq2, rads = self._potential_tables()
-        self.utility_border = ub
+        self.utility_border = copy.deepcopy(ub)   # the caller's to change; the tables' own is not
         # the absorptive correction of the dyadic Green's function (:322)
         a2 = F32((2 * math.pi * ub.k0_nm) ** 2)
         absorb = C64(a2 / C64(a2 + 1j * self.eps_imag))
