@@ -268,7 +268,8 @@ struct FineButterfly<3, INV> {
     const float lo = (float)(0.875 - 0.86602540378443864676);
     const float2 x0 = v[0], a = cadd(v[1], v[2]);
     // j = -/+ i (v1 - v2)
-    const float2 j = INV ? make_float2(v[2].y - v[1].y, v[1].x - v[2].x) : make_float2(v[1].y - v[2].y, v[2].x - v[1].x);
+    const float2 j =
+        INV ? make_float2(v[2].y - v[1].y, v[1].x - v[2].x) : make_float2(v[1].y - v[2].y, v[2].x - v[1].x);
     const float2 m = cfma_real(-0.5f, a, x0);
     v[0] = cadd(x0, a);
     v[1] = cfma_real(-lo, j, cfma_real(0.875f, j, m));
@@ -282,8 +283,11 @@ struct FineButterfly<5, INV> {
     const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
     const float s2 = 0.58778525229247312917f, lo = (float)(1 - 0.95105651629515357212);
     const float2 x0 = v[0], a1 = cadd(v[1], v[4]), a2 = cadd(v[2], v[3]);
-    const float2 j1 = INV ? make_float2(v[4].y - v[1].y, v[1].x - v[4].x) : make_float2(v[1].y - v[4].y, v[4].x - v[1].x);
-    const float2 j2 = INV ? make_float2(v[3].y - v[2].y, v[2].x - v[3].x) : make_float2(v[2].y - v[3].y, v[3].x - v[2].x);
+    // j = -/+ i (v[m] - v[5 - m])
+    const float2 j1 =
+        INV ? make_float2(v[4].y - v[1].y, v[1].x - v[4].x) : make_float2(v[1].y - v[4].y, v[4].x - v[1].x);
+    const float2 j2 =
+        INV ? make_float2(v[3].y - v[2].y, v[2].x - v[3].x) : make_float2(v[2].y - v[3].y, v[3].x - v[2].x);
     const float2 p1 = cfma_real(c2, a2, cfma_real(c1, a1, x0)), p2 = cfma_real(c1, a2, cfma_real(c2, a1, x0));
     const float2 q1 = cfma_real(-lo, j1, cfma_real(s2, j2, j1));               // sin(2 pi / 5) j1 + s2 j2
     const float2 q2 = cfma_real(lo, j2, csub(cscale(j1, s2), j2));             // s2 j1 - sin(2 pi / 5) j2
@@ -304,7 +308,8 @@ struct FineButterfly<8, INV> {
     Butterfly<4, INV>::run(e, nullptr, 0);
     Butterfly<4, INV>::run(o, nullptr, 0);
     // as Butterfly<8>: o1 and o3 hold W8^k o[k] sqrt(2)
-    const float2 o1 = INV ? make_float2(o[1].x - o[1].y, o[1].x + o[1].y) : make_float2(o[1].x + o[1].y, o[1].y - o[1].x);
+    const float2 o1 =
+        INV ? make_float2(o[1].x - o[1].y, o[1].x + o[1].y) : make_float2(o[1].x + o[1].y, o[1].y - o[1].x);
     const float2 o3 =
         INV ? make_float2(-(o[3].x + o[3].y), o[3].x - o[3].y) : make_float2(o[3].y - o[3].x, -(o[3].x + o[3].y));
     v[0] = cadd(e[0], o[0]);
@@ -409,24 +414,27 @@ ODT_ODD_BUTTERFLY(31)
 // for the short constants of the 8-point step beside it (Born series on padded
 // 160 x 160 x 96, rounding against double precision: 0.80e-7, with the split
 // one 0.96e-7).
+// The larger factor goes first: the other way round the compiler keeps far more
+// values at once (z passes of 21 points: 352 and 1864 bytes of spills a thread
+// against 12 and none; 44 x 44 x 147 padded dyadic solve 2.15 against 1.64 ms).
 #define ODT_COMPOSITE_BUTTERFLY(A, B) ODT_COMPOSITE_BUTTERFLY_OF(A, B, FineButterfly)
-ODT_COMPOSITE_BUTTERFLY(2, 3)
-ODT_COMPOSITE_BUTTERFLY_OF(2, 5, Butterfly)
+ODT_COMPOSITE_BUTTERFLY(3, 2)
+ODT_COMPOSITE_BUTTERFLY_OF(5, 2, Butterfly)
 ODT_COMPOSITE_BUTTERFLY(4, 3)
-ODT_COMPOSITE_BUTTERFLY(2, 7)
-ODT_COMPOSITE_BUTTERFLY(3, 5)
+ODT_COMPOSITE_BUTTERFLY(7, 2)
+ODT_COMPOSITE_BUTTERFLY(5, 3)
 ODT_COMPOSITE_BUTTERFLY(4, 4)
-ODT_COMPOSITE_BUTTERFLY(2, 9)
-ODT_COMPOSITE_BUTTERFLY_OF(4, 5, Butterfly)
-ODT_COMPOSITE_BUTTERFLY(3, 7)
-ODT_COMPOSITE_BUTTERFLY(2, 11)
-ODT_COMPOSITE_BUTTERFLY(3, 8)
+ODT_COMPOSITE_BUTTERFLY(9, 2)
+ODT_COMPOSITE_BUTTERFLY_OF(5, 4, Butterfly)
+ODT_COMPOSITE_BUTTERFLY(7, 3)
+ODT_COMPOSITE_BUTTERFLY(11, 2)
+ODT_COMPOSITE_BUTTERFLY(8, 3)
 ODT_COMPOSITE_BUTTERFLY(5, 5)
-ODT_COMPOSITE_BUTTERFLY(2, 13)
+ODT_COMPOSITE_BUTTERFLY(13, 2)
 ODT_COMPOSITE_BUTTERFLY(3, 9)
-ODT_COMPOSITE_BUTTERFLY(4, 7)
-ODT_COMPOSITE_BUTTERFLY_OF(5, 6, Butterfly)
-ODT_COMPOSITE_BUTTERFLY_OF(5, 7, Butterfly)
+ODT_COMPOSITE_BUTTERFLY(7, 4)
+ODT_COMPOSITE_BUTTERFLY(10, 3)
+ODT_COMPOSITE_BUTTERFLY_OF(7, 5, Butterfly)
 #undef ODT_COMPOSITE_BUTTERFLY
 
 // ------------------------------------------------------------------ one pass
