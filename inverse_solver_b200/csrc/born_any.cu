@@ -1,14 +1,17 @@
-// Born loop for padded grids with a length that the radix tiles do not cover
-// (a prime factor above 31: the reference pads the RI grid by the boundary
+// Pointwise passes for padded grids with a length that the radix tiles do not
+// cover (a prime factor above 31: the reference pads the RI grid by the boundary
 // width without rounding, FORWARD_SOLVER_CONVERGENT_BORN.m:129, so any
-// length occurs).  The transforms along such an axis run through Bluestein's
-// algorithm (fft_any.cu), so the Born iteration is unfused here: per
-// iteration jj
+// length occurs).  The transforms along such an axis are kernels of their own:
+// direct products (prime_pass.cu) where they apply, with the z-pass in one
+// kernel, else Bluestein's algorithm (fft_any.cu).  born_point is the x-pass's
+// pointwise work between the transforms of such an x-axis.  Where the z-axis has
+// no kernel of its own (Bluestein), and for ODT_KERNELS=generic, the whole
+// iteration is unfused: per iteration jj
 //   born_point  the inverse transform's result in T -> update of iteration
 //               jj-1 (:616-642) and the source of jj times the phase ramp
 //               (:588-605) back into T (the generic x-pass's pointwise work,
 //               BornXOp, one element per thread);
-//   3D FFT      forward along x, y, z (tile kernels or Bluestein per axis);
+//   3D FFT      forward along x, y, z (tile kernels, direct products or Bluestein per axis);
 //   born_green  G(k -/+ dk/4) / N (:606-615, the generic z-pass's GreenOp);
 //   3D FFT      inverse along z, y, x (unnormalised: 1/N is in born_green).
 #include <cuda_runtime.h>

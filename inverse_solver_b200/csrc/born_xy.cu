@@ -9,8 +9,9 @@
 //   transforms of PSI = ifftn(G .* fftn(psi)) of iteration jj-1), update of
 //   iteration jj-1 (:616-642), source term of iteration jj times the phase
 //   ramp (:588-605), forward x-FFT and forward y-FFT (the first two of fftn).
-// The z-pass (cols_pipe.cu) does the z-FFT, the Green's multiply and the
-// inverse z-FFT in between.
+// The z-pass (z_pass.cu, z_dyadic.cu, prime_pass.cu or the generic tiles; 16-bit
+// storage: cols_pipe.cu) does the z-FFT, the Green's multiply and the inverse z-FFT
+// in between.
 //
 // Transforms along an axis of length N = 8 R (5 <= R <= 28): index
 // n = R n1 + n2 (n1 < 8, n2 < R), k = k1 + 8 k2 (k1 < 8, k2 < R).

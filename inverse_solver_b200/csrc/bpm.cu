@@ -523,7 +523,7 @@ cudaError_t run_lines_c(float2* fld, const PhaseOp& op, const DevFft& f, int las
   const size_t sm = align16(sizeof(float2) * f.plan.n) + 2 * sizeof(float2) * (size_t)W * smem_line_ld(f.plan.n);
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(bpm_lines_kernel<CLS>), sm);
   if (e != cudaSuccess) return e;
-  return launch_pdl(bpm_lines_kernel<CLS>, 1, (unsigned)((op.nlines + W - 1) / W), kTileThreads, sm, s, fld, op, f.plan,
+  return launch_pdl(bpm_lines_kernel<CLS>, (unsigned)((op.nlines + W - 1) / W), kTileThreads, sm, s, fld, op, f.plan,
                     f.tw, W, last);
 }
 cudaError_t run_lines(float2* fld, const PhaseOp& op, const DevFft& f, int last, cudaStream_t s) {
@@ -536,7 +536,7 @@ cudaError_t run_cols_c(float2* fld, const float2* rk, int n1, int nill, const De
   const size_t sm = align16(sizeof(float2) * f.plan.n) + 2 * sizeof(float2) * (size_t)f.plan.n * (W + 1);
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(bpm_cols_kernel<CLS>), sm);
   if (e != cudaSuccess) return e;
-  return launch_pdl(bpm_cols_kernel<CLS>, 1, (unsigned)((n1 + W - 1) / W) * nill, kTileThreads, sm, s, fld, rk, n1, f.plan,
+  return launch_pdl(bpm_cols_kernel<CLS>, (unsigned)((n1 + W - 1) / W) * nill, kTileThreads, sm, s, fld, rk, n1, f.plan,
                     f.tw, lg);
 }
 cudaError_t run_cols(float2* fld, const float2* rk, int n1, int nill, const DevFft& f, cudaStream_t s) {

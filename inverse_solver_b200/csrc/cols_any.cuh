@@ -22,21 +22,15 @@ constexpr int kThreads = 160;
 constexpr int kMaxN = 256;      // rows of a TMA box
 constexpr int kMaxR = 31;
 
-constexpr bool has_radix(int r) {   // as a register butterfly
-  return r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 7 || r == 8 || r == 9 || r == 10 || r == 11 ||
-         r == 12 || r == 13 || r == 14 || r == 15 || r == 16 || r == 17 || r == 18 || r == 19 || r == 20 ||
-         r == 21 || r == 22 || r == 23 || r == 24 || r == 25 || r == 26 || r == 27 || r == 28 || r == 29 ||
-         r == 30 || r == 31;
-}
 // A of n = A R (0: none): 8 where it divides (kernels of their own, whose
 // registers no other factor shares), else the largest A <= 10, else the
 // smallest above
 constexpr int z_split(int n) {
   if (n % 8 == 0 && n / 8 >= 8 && n / 8 <= kMaxR) return 8;
   for (int A = 10; A >= 2; --A)
-    if (n % A == 0 && n / A >= A && n / A <= kMaxR && has_radix(n / A)) return A;
+    if (n % A == 0 && n / A >= A && n / A <= kMaxR) return A;
   for (int A = 11; A <= 16; ++A)
-    if (n % A == 0 && n / A >= A && n / A <= kMaxR && has_radix(n / A)) return A;
+    if (n % A == 0 && n / A >= A && n / A <= kMaxR) return A;
   return 0;
 }
 

@@ -110,8 +110,8 @@ struct Handle {
 
   // transform lengths
   DevFft fx{}, fy{}, fz{}, ffx{}, ffy{}, fcx{}, fcy{};
-  // Bluestein plans of the lengths the radix tiles do not cover (direct =
-  // true for the others; the DevFft of such a length has no passes)
+  // plans (direct products or Bluestein) of the lengths the radix tiles do not
+  // cover (direct = true for the others; the DevFft of such a length has no passes)
   AnyFft bsx{}, bsy{}, bsz{}, bsfx{}, bsfy{}, bscx{}, bscy{};
   bool any_loop() const { return !bsx.direct || !bsy.direct || !bsz.direct; }
   bool any_io() const { return !bsfx.direct || !bsfy.direct || !bscx.direct || !bscy.direct; }

@@ -18,22 +18,17 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
-cudaError_t launch_pdl(void (*kernel)(P...), int cluster, unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                       A&&... args) {
-  cudaLaunchAttribute at[2];
+cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = (unsigned)cluster;
-  at[1].val.clusterDim.y = 1;
-  at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
