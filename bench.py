@@ -715,7 +715,7 @@ def main():
     ap.add_argument("--fista", action="store_true",
                     help="time FISTA outer iterations of the inverse solver (device vs host loop)")
     ap.add_argument("--grid-lengths", nargs="*", type=int, default=None, metavar="RI_SIZE",
-                    help="time the Born loop on padded grids of 96^3, 127^3 (Bluestein), 128^3, 136^3, 152^3 "
+                    help="time the Born loop on padded grids of 96^3, 127^3 (prime), 128^3, 136^3, 152^3 "
                          "and 160^3 (RI sizes 72, 103, 104, 112, 128, 136; give some of them to time only those)")
     ap.add_argument("--print-rank-env", action="store_true",
                     help="print each rank's RANK / LOCAL_RANK / WORLD_SIZE and exit (launcher check)")

@@ -13,8 +13,8 @@
 // X_(p-k) and multiplies them by the Green's function on the way back to
 // shared memory.
 //
-// What bounds it: issue latency at 16 warps per SM (128 registers); the FMA
-// pipe is busy 35 to 40 %.  The coefficients in shared memory and a second
+// What bounds it: issue latency at 16 warps per SM (128 registers); in the
+// z-pass the FMA pipe is busy 55 % and the issue slots 57 %.  The coefficients in shared memory and a second
 // landing stage (8 warps per SM) measured 0.38 ms, one stage with 4 pencils per
 // thread 0.34 with half the speed for q > 1, pairs of k in the packed
 // multiply-adds 0.40, against 0.34 ms for a 127-point axis of 16 x 127^3 as

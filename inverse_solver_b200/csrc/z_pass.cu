@@ -22,8 +22,13 @@
 // items (one round of the 160 threads), and the larger radix sits in registers
 // between two transforms.
 //
-// What bounds it: the steps' instructions and the two barriers between them,
-// not DRAM (16 bytes per element).
+// What bounds it: the steps' instructions and the two barriers between them
+// (153 points: issue slots 53 % busy, barrier the first of the stalls), not DRAM
+// (16 bytes per element, 27 % of its rate).  The kernels of A != 8 spill at large odd R
+// under their launch bounds: 212 bytes stored a thread at 17, 260 at 19, 372 at 23,
+// 500 at 29, 596 at 31.  The correctly rounded reciprocal of the Green's function
+// costs 8 % of a pass of 152 points (0.67 -> 0.73 ms, 49 illuminations) over the
+// hardware's approximation with a refinement.
 #include <type_traits>
 
 #include "cols_any.cuh"
