@@ -14,11 +14,11 @@
 // shared memory.
 //
 // What bounds it: issue latency at 16 warps per SM (128 registers); in the
-// z-pass the FMA pipe is busy 55 % and the issue slots 57 %.  The coefficients in shared memory and a second
-// landing stage (8 warps per SM) measured 0.38 ms, one stage with 4 pencils per
-// thread 0.34 with half the speed for q > 1, pairs of k in the packed
-// multiply-adds 0.40, against 0.34 ms for a 127-point axis of 16 x 127^3 as
-// it stands.  One Bluestein kernel per axis and direction (two transforms of
+// z-pass the FMA pipe is busy 55 % and the issue slots 57 %.  The coefficients
+// in shared memory and a second landing stage (8 warps per SM) measured 0.38 ms,
+// one stage with 4 pencils per thread 0.34 with half the speed for q > 1, pairs of k
+// in the packed multiply-adds 0.40, against 0.34 ms for a 127-point axis of
+// 16 x 127^3 as it stands.  One Bluestein kernel per axis and direction (two transforms of
 // m >= 2 p - 1 points and two chirps through shared memory) took 0.58 ms, and
 // the z-pass as two of those and a separate product 1.34 against 0.60 ms.
 //
@@ -29,7 +29,8 @@
 // with ideal inner transforms.  Above p = 139 the sums therefore run in two
 // halves: 1.2e-7 (151), 1.4e-7 (211), 1.55e-7 (251), for 3 to 14 % of the axis's time
 // (20 M points, lines and columns: 151 points 0.280 -> 0.289 and 0.252 -> 0.287 ms, 251
-// points 0.365 -> 0.387 and 0.324 -> 0.351).  FP32 throughout; tcgen05 has no FP32
+// points 0.365 -> 0.387 and 0.324 -> 0.351) and 12 to 21 % of a z-pass's, which holds two
+// such sums (36 x 40 x 149, 8 waves: 0.054 -> 0.060 ms, x 251: 0.116 -> 0.140).  FP32 throughout; tcgen05 has no FP32
 // multiply, and its TF32 form would need the operands in three parts.
 #include <cmath>
 #include <type_traits>
